@@ -1387,16 +1387,33 @@ int hfg_eri_gradient(hfg_ctx* ctx, double schwarz_threshold, int nspin, const do
   a.Dspin = ctx->d_Ds.p;
   a.n = ctx->n;
   a.nspin = nspin;
-  for (size_t l = 0; l < plan->launches.size(); ++l) {
+  // the classes run concurrently over the context stream and its side
+  // streams (each adds into the gradient with atomics)
+  HFG_CUDA(ctx, ctx->ensure_side_streams());
+  HFG_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
+  for (int k = 0; k < kJKSideStreams; ++k) HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
+  cudaError_t le = cudaSuccess;
+  for (size_t l = 0; l < plan->launches.size() && le == cudaSuccess; ++l) {
     const Launch& L = plan->launches[l];
     a.counter = ctx->d_counters.p + l;
     a.entries = L.d_entries;
     a.prefix = L.d_prefix;
+    a.nentries = (int)L.prefix[0];
+    a.nwarps = L.prefix[1];
     a.chunk_entry = L.d_chunk;
     a.chunk_start = L.d_cstart;
     a.nchunks = L.nchunks;
-    HFG_CUDA(ctx, launch_grad_md(L.la, L.lb, L.lc, L.ld, a, d_atom.p, d_grad.p, ctx->stream));
+    const size_t si = l % (1 + kJKSideStreams);
+    le = launch_eri_gradient(L.la, L.lb, L.lc, L.ld, a, d_atom.p, natom, d_grad.p,
+                             si == 0 ? ctx->stream : ctx->side[si - 1]);
   }
+  // the side streams are joined on every path: the buffers below are
+  // released in the order of the context stream
+  for (int k = 0; k < kJKSideStreams; ++k) {
+    HFG_CUDA(ctx, cudaEventRecord(ctx->ev_join[k], ctx->side[k]));
+    HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_join[k], 0));
+  }
+  HFG_CUDA(ctx, le);
   HFG_CUDA(ctx, cudaMemcpyAsync(grad, d_grad.p, (size_t)3 * natom * sizeof(double), cudaMemcpyDeviceToHost,
                                 ctx->stream));
   HFG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
