@@ -17,7 +17,6 @@ struct MDClass {
 };
 
 MDClass md_class(int la, int lb, int lc, int ld);
-size_t md_smem_bytes(const MDClass& c);
 bool md_class_ok(int la, int lb, int lc, int ld);
 
 cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,
