@@ -385,18 +385,107 @@ static int build_pairs(hfg_ctx* ctx) {
   return HFG_OK;
 }
 
+// Nominal primitive quartets per lane of one warp task of an entry.
+static double entry_cost(const hfg_ctx* ctx, const JKEntry& x) {
+  return (double)prim_range(0, 1, ctx->h_pairs[x.bra].npp, x.slice, 0).count *
+         prim_range(0, 1, ctx->h_pairs[x.k_lo].npp, x.slice, 16).count;
+}
+
+// Whether a launch runs on the block-per-quartet engine instead of its
+// generated kernel: FP64 launches of few quartets in the classes with L >= 5,
+// whose straight-line code (up to 1 MB) takes 0.1 to 0.7 ms to pass through
+// once, however few quartets there are.  Measured on water clusters of 1 to
+// 32 molecules, limits of 0 / 500 / 2,000 / 8,000 quartets: one water 842 /
+// 255 / 257 / 259 us, (H2O)4 1,808 / 1,162 / 1,224 / 1,906 us, mixed (H2O)32
+// 108.9 / 109.4 / 113.2 / 113.1 ms.  A batched launch has its quartets spread
+// over many short queues and gains up to 2,000 (4.78 ms at 500, 4.57 at 2,000,
+// 4.96 at 8,000 for 48 molecules of 1 to 4 waters), and so does the packed
+// tensor, whose kernels do not split the heavy classes' quartets.
+static bool coop_launch(const Launch& L, PlanUse use) {
+  const double limit = use == kPlanBatch || use == kPlanWhole ? 2000.0 : 500.0;
+  return !L.fp32 && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
+}
+
+// Splits the entries whose lanes (or, on the block-per-quartet engine, whose
+// blocks) would walk more primitive quartets than their share of the launch
+// over sms x 16 warps: a (ss|ss) quartet of 8 x 8 primitives each walks 4,096
+// one after another, 1.2 ms, while a molecule of a few atoms fills a fraction
+// of the GPU.  J and K are linear in the integrals, so a slice is digested
+// like a quartet, and the digestion bounds the slices from below at 32
+// primitive quartets (8 / 16 / 32 / 64: one water in cc-pVDZ 214 / 219 / 214 /
+// 263 us, (H2O)5 1,943 / 1,867 / 1,826 / 1,786, (H2O)5 in STO-3G, UHF, 216 /
+// 135 / 100 / 124).  Batched builds fill the GPU with whole molecules and
+// slice from 128.  FP32 launches hold
+// quartets with few primitive quartets left and are not sliced.
+static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sms, PlanUse use) {
+  const bool generic = L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
+  if (L.fp32 || use == kPlanWhole || (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld))) return false;
+  const bool block = use == kPlanGrad || (use == kPlanJK && (L.coop || generic));  // a block per quartet
+  double total = 0.0;
+  for (const JKEntry& x : L.entries) total += entry_cost(ctx, x) * (block ? x.k_hi - x.k_lo : (x.k_hi - x.k_lo + 31) / 32);
+  double target;
+  if (block) target = std::max(2.0, total / ((double)sms * md_blocks_per_sm(L.la, L.lb, L.lc, L.ld)));
+  else if (use == kPlanBatch) target = std::max(128.0, total / ((double)sms * 16));
+  else target = std::max(32.0, total / ((double)sms * 16));
+  std::vector<JKEntry> out;
+  bool any = false;
+  for (const JKEntry& x : L.entries) {
+    const PairInfo &b = ctx->h_pairs[x.bra], &k = ctx->h_pairs[x.k_lo];
+    if ((double)b.npp * k.npp <= target) {
+      out.push_back(x);
+      continue;
+    }
+    // primitive quartets of the first ket that survive screening (bounds are
+    // sorted, so the bra count falls as the ket index grows)
+    const PrimPair *pb = ctx->h_prims.data() + b.pp_off, *pk = ctx->h_prims.data() + k.pp_off;
+    int eb = b.npp, ek = 0, nb = b.npp;
+    double eff = 0.0;
+    for (int q = 0; q < k.npp; ++q) {
+      while (nb > 0 && pb[nb - 1].bound * pk[q].bound < prim_eps) --nb;
+      if (q == 0) eb = nb;
+      if (nb == 0) break;
+      ++ek;
+      eff += nb;
+    }
+    const double want = std::ceil(eff / target);
+    const int sb = std::max(1, std::min({eb, 255, (int)want}));
+    const int sk = std::max(1, std::min({ek, 255, (int)std::ceil(want / sb)}));
+    if (sb * sk == 1) {
+      out.push_back(x);
+      continue;
+    }
+    any = true;
+    for (int i = 0; i < sb; ++i)
+      for (int j = 0; j < sk; ++j) {
+        JKEntry y = x;
+        y.slice = (unsigned)i | (unsigned)sb << 8 | (unsigned)j << 16 | (unsigned)sk << 24;
+        out.push_back(y);
+      }
+  }
+  L.entries.swap(out);
+  return any;
+}
+
 // Launch plan for (Schwarz threshold, FP32 threshold, precision): for every
 // pair of pair classes (bra class >= ket class) and every bra pair, the
 // significant kets form a prefix of the ket class (kets sorted by Q); in
 // mixed precision the kets below the FP32 threshold form the tail of it.
-static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, int precision, int tile,
+static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, int precision, int tile, PlanUse use,
                       Plan*& out) {
   if (tile <= 0) tile = 64;
   auto key = std::make_tuple(thr, precision == HFG_MIXED ? mixed : 0.0, prim_eps, precision, tile);
   auto it = ctx->plans.find(key);
-  if (it != ctx->plans.end()) {
+  if (it != ctx->plans.end() && (use == kPlanJK || !it->second->sliced)) {
     out = it->second.get();
     return HFG_OK;
+  }
+  hfg_ctx::PlanMap& mine = use == kPlanJK ? ctx->plans : ctx->other_plans[use - 1];
+  if (use != kPlanJK) {
+    it = mine.find(key);
+    if (it != mine.end()) {
+      out = it->second.get();
+      return HFG_OK;
+    }
   }
   auto plan = std::make_unique<Plan>();
   std::map<std::tuple<int, int, int, int, int>, int> lidx;
@@ -473,10 +562,20 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   std::sort(plan->launches.begin(), plan->launches.end(), [](const Launch& x, const Launch& y) {
     return std::make_tuple(x.la + x.lb + x.lc + x.ld, x.fp32) > std::make_tuple(y.la + y.lb + y.lc + y.ld, y.fp32);
   });
+  // The launches of a large plan fill the GPU one by one, and more of them at
+  // once only share its caches (eight streams / four: (H2O)5 in cc-pVDZ 1,925
+  // / 2,051 us, (H2O)12 in 6-31G* 3,109 / 3,178 us; (H2O)12 in cc-pVDZ 21.8 /
+  // 21.4 ms, mixed UHF (H2O)24 73.3 / 70.8 ms): four from 2.5e7
+  // quartets, (H2O)12 in cc-pVDZ.
+  double quartets = 0.0;
+  for (const Launch& L : plan->launches) quartets += L.quartets;
+  if (quartets > 2.5e7) plan->streams = 4;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   for (auto& L : plan->launches) {
     L.st = ctx->stream;
+    L.coop = coop_launch(L, use);
+    if (slice_entries(ctx, L, prim_eps, sms, use)) plan->sliced = true;
     // Work-queue steps.  Entries are ordered by the nominal cost of one of
     // their warp tasks (bra x ket primitive pairs, before primitive
     // screening), most expensive first, so that the cheap tasks form the
@@ -490,7 +589,7 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
       const size_t ne = L.entries.size();
       cost.resize(ne);
       for (size_t e = 0; e < ne; ++e)
-        cost[e] = (double)ctx->h_pairs[L.entries[e].bra].npp * ctx->h_pairs[L.entries[e].k_lo].npp;
+        cost[e] = entry_cost(ctx, L.entries[e]);
       std::vector<size_t> ord(ne);
       std::iota(ord.begin(), ord.end(), 0);
       std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return cost[x] > cost[y]; });
@@ -559,7 +658,7 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   st.launches = (int)plan->launches.size();
   plan->stats = st;
   out = plan.get();
-  ctx->plans[key] = std::move(plan);
+  mine[key] = std::move(plan);
   return HFG_OK;
 }
 
@@ -694,7 +793,7 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
   if (ctx->batcher && nspin == 1 && nshards == 1 && dPs == dPt && !o.deterministic)
     return batcher_submit(ctx->batcher, ctx, o, dPt, dJ, dK);
   Plan* plan = nullptr;
-  int rc = build_plan(ctx, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile, plan);
+  int rc = build_plan(ctx, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile, kPlanJK, plan);
   if (rc != HFG_OK) return rc;
   const size_t nn = (size_t)ctx->n * ctx->n;
   HFG_CUDA(ctx, ctx->d_Jacc.alloc(nn));
@@ -769,13 +868,13 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
   // they are spread over the context stream and its side streams so that
   // they run concurrently (parallel branches when captured into a graph).  A
   // small molecule's build then costs about its slowest class instead of the
-  // sum over classes; a large one's persistent grids fill the GPU either way.
-  // Profiled builds stay on one stream (per-launch events).
-  const int nstreams = (profile || a.serial) ? 1 : 1 + kJKSideStreams;
+  // sum over classes; a large one's persistent grids fill the GPU either way
+  // (plan->streams).  Profiled builds stay on one stream (per-launch events).
+  const int nstreams = (profile || a.serial) ? 1 : plan->streams;
   if (nstreams > 1) {
     HFG_CUDA(ctx, ctx->ensure_side_streams());
     HFG_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
-    for (int k = 0; k < kJKSideStreams; ++k) HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
+    for (int k = 0; k < nstreams - 1; ++k) HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
   }
   for (size_t l = 0; l < plan->launches.size(); ++l) {
     const Launch& L = plan->launches[l];
@@ -804,11 +903,11 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
     a.nchunks = c1 - c0;
     a.nentries = (int)L.prefix[0];
     a.nwarps = L.prefix[1];
-    HFG_CUDA(ctx, launch_jk(L.la, L.lb, L.lc, L.ld, L.fp32, a, ls));
+    HFG_CUDA(ctx, launch_jk(L.la, L.lb, L.lc, L.ld, L.fp32, L.coop, a, ls));
     if (profile) cudaEventRecord(ev[l + 1], ctx->stream);
   }
   if (nstreams > 1) {
-    for (int k = 0; k < kJKSideStreams; ++k) {
+    for (int k = 0; k < nstreams - 1; ++k) {
       HFG_CUDA(ctx, cudaEventRecord(ctx->ev_join[k], ctx->side[k]));
       HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_join[k], 0));
     }
@@ -872,13 +971,14 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
 }  // namespace hfg
 
 hfg_ctx::~hfg_ctx() {
-  for (auto& kv : plans)
-    for (auto& L : kv.second->launches) {
-      if (L.d_entries) cudaFreeAsync(L.d_entries, L.st);
-      if (L.d_prefix) cudaFreeAsync(L.d_prefix, L.st);
-      if (L.d_chunk) cudaFreeAsync(L.d_chunk, L.st);
-      if (L.d_cstart) cudaFreeAsync(L.d_cstart, L.st);
-    }
+  for (auto* map : {&plans, &other_plans[0], &other_plans[1], &other_plans[2]})
+    for (auto& kv : *map)
+      for (auto& L : kv.second->launches) {
+        if (L.d_entries) cudaFreeAsync(L.d_entries, L.st);
+        if (L.d_prefix) cudaFreeAsync(L.d_prefix, L.st);
+        if (L.d_chunk) cudaFreeAsync(L.d_chunk, L.st);
+        if (L.d_cstart) cudaFreeAsync(L.d_cstart, L.st);
+      }
   for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
   // every device buffer is released here, before the context's stream is
   // destroyed (their frees are ordered on it)
@@ -1169,7 +1269,7 @@ int jk_batch_locked(hfg_ctx* const* ctxs, int n_jobs, const hfg_jk_opts* opts, c
     AllocScope alloc_scope(c->stream);
     const hfg_jk_opts& o = opts[j];
     const int rc =
-        build_plan(c, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile, plans[j]);
+        build_plan(c, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile, kPlanBatch, plans[j]);
     if (rc != HFG_OK) return fail(rc, c->err);
     const size_t nn = (size_t)c->n * c->n;
     BK(c->d_Jacc.alloc(nn));
@@ -1179,7 +1279,7 @@ int jk_batch_locked(hfg_ctx* const* ctxs, int n_jobs, const hfg_jk_opts* opts, c
         BK(c->d_D32.alloc(3 * nn));
         break;
       }
-    BK(c->ensure_side_streams());
+    BK(j == 0 ? c->ensure_side_streams() : c->ensure_fork());
     if (c->stream != st) {
       BK(cudaEventRecord(c->ev_fork, c->stream));
       BK(cudaStreamWaitEvent(st, c->ev_fork, 0));
@@ -1312,8 +1412,16 @@ int jk_batch_locked(hfg_ctx* const* ctxs, int n_jobs, const hfg_jk_opts* opts, c
     a.job_steps = reinterpret_cast<const long long*>(dev + steps_off[g]);
     a.njobs = (int)glist[g].second->size();
     a.nchunks = total[g];
+    // (the total over the molecules decides, not each one's own)
+    Launch sum{};
+    sum.la = la;
+    sum.lb = lb;
+    sum.lc = lc;
+    sum.ld = ld;
+    sum.fp32 = f32 != 0;
+    for (const Member& m : *glist[g].second) sum.quartets += m.L->quartets;
     const int si = g % nstreams;
-    BK(launch_jk_batch(la, lb, lc, ld, f32 != 0, a, si == 0 ? st : c0->side[si - 1]));
+    BK(launch_jk_batch(la, lb, lc, ld, f32 != 0, coop_launch(sum, kPlanBatch), a, si == 0 ? st : c0->side[si - 1]));
   }
   for (int k = 0; k < kJKSideStreams; ++k) {
     BK(cudaEventRecord(c0->ev_join[k], c0->side[k]));
@@ -1360,7 +1468,7 @@ int hfg_eri_gradient(hfg_ctx* ctx, double schwarz_threshold, int nspin, const do
     for (int k = 0; k < ncart(sh.l); ++k) ao_atom[sh.ao + k] = sh.atom;
   }
   Plan* plan = nullptr;
-  int rc = build_plan(ctx, schwarz_threshold, 0.0, 0.0, HFG_FP64, 0, plan);
+  int rc = build_plan(ctx, schwarz_threshold, 0.0, 0.0, HFG_FP64, 0, kPlanGrad, plan);
   if (rc != HFG_OK) return rc;
   const size_t nn = (size_t)ctx->n * ctx->n;
   HFG_CUDA(ctx, ctx->d_D.alloc(nn));
@@ -1466,7 +1574,7 @@ int eri_packed_locked(hfg_ctx* ctx, double thr, double* d_out, size_t len) {
     return set_error(ctx, HFG_ERR_INVALID_INPUT, "packed length must be n_p (n_p + 1) / 2 with n_p = n (n + 1) / 2");
   if (!(thr >= 0.0)) return set_error(ctx, HFG_ERR_INVALID_INPUT, "Schwarz threshold must be >= 0");
   Plan* plan = nullptr;
-  int rc = build_plan(ctx, thr, 0.0, 0.0, HFG_FP64, 0, plan);
+  int rc = build_plan(ctx, thr, 0.0, 0.0, HFG_FP64, 0, kPlanWhole, plan);
   if (rc != HFG_OK) return rc;
   HFG_CUDA(ctx, cudaMemsetAsync(d_out, 0, len * sizeof(double), ctx->stream));
   for (const Launch& L : plan->launches) {

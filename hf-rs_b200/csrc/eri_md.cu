@@ -37,12 +37,14 @@ namespace {
 constexpr int kMDThreads = 512;  // largest block
 constexpr int kMDAcc = 20;       // output elements per thread, at most
 
-// Threads by the number of block elements: enough that each holds at most
-// kMDAcc of them ((ff|ff): 10,000 / 512), and no more, since the per-primitive
-// steps of the small classes are shorter than a barrier of a wide block.
+// Threads by the number of items of four block elements: enough that each
+// holds at most kMDAcc elements ((ff|ff): 2,500 items over 512), and no more,
+// since the per-primitive steps of the small classes are shorter than a
+// barrier of a wide block.
+__host__ __device__ inline int md_items(const MDClass& c) { return (c.na * c.nb + 3) / 4 * c.nc * c.nd; }
 __host__ __device__ inline int md_threads(const MDClass& c) {
-  const int n = c.na * c.nb * c.nc * c.nd;
-  return n <= 128 ? 32 : (n <= 512 ? 64 : (n <= 1536 ? 128 : (n <= 4096 ? 256 : 512)));
+  const int n = md_items(c);
+  return n <= 32 ? 32 : (n <= 128 ? 64 : (n <= 384 ? 128 : (n <= 1024 ? 256 : 512)));
 }
 
 // Density blocks of one quartet's digestion: D[cd], D[ab], then per spin
@@ -56,6 +58,8 @@ __host__ __device__ inline int md_dsize(const MDClass& c) {
 // and the density blocks.
 struct MDShared {
   int nab, ncd, gs, os;  // gs, os: odd row strides of G[k][ab] and out[cd][ab]
+  int na4;               // a thread's elements of one cd are ab, ab + na4, ab + 2 na4, ab + 3 na4
+  float inv_na4;
   double *S, *G, *out, *D;
   coop::Side B, K;
   coop::RTab R;
@@ -76,6 +80,8 @@ __device__ void md_setup(const MDClass& c, unsigned char* raw, MDShared& s) {
   s.nab = c.na * c.nb;
   s.ncd = c.nc * c.nd;
   s.gs = s.os = s.nab | 1;
+  s.na4 = (s.nab + 3) / 4;
+  s.inv_na4 = 1.0f / s.na4;
   s.S = reinterpret_cast<double*>(raw);
   unsigned char* p = raw + 64;
   s.G = s.out = reinterpret_cast<double*>(p);
@@ -118,18 +124,18 @@ struct PrimRecs {
   __device__ __forceinline__ float bound(int k) const { return pbound[off + k * stride]; }
 };
 
-// The contracted block of nb x nk primitive pairs, element x = cd nab + ab
-// of thread x % nt in acc[x / nt]; primitive quartets with bound products
+// The contracted block of nb x nk primitive pairs in acc, four elements
+// (cd; ab, ab + na4, ...) per item cd na4 + ab of thread item % nt; primitive quartets with bound products
 // below eps are skipped (eps = 0: none).  The R tables' index list is made
 // here, since a finished block overwrites it.
 template <int ACC, typename PB, typename PK>
 __device__ __forceinline__ void md_quartet(const MDShared& s, const PB& pb, int nb, const PK& pk, int nk,
                                            const double* AB, const double* CD, const double* AC, double eps,
-                                           const double* __restrict__ boys, const double* __restrict__ expt,
+                                           const double* __restrict__ boys,
                                            double (&acc)[ACC]) {
   const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-  const int nh = s.K.nh, n = s.nab * s.ncd;
-  const float inv_nh = 1.0f / nh, inv_nab = 1.0f / s.nab, feps = (float)eps;
+  const int nh = s.K.nh, nq = (nh + 3) / 4;
+  const float inv_nq = 1.0f / nq, feps = (float)eps;
 #pragma unroll
   for (int i = 0; i < ACC; ++i) acc[i] = 0.0;
   __syncthreads();  // the previous block has been read
@@ -151,15 +157,10 @@ __device__ __forceinline__ void md_quartet(const MDShared& s, const PB& pb, int 
           const double PQ[3] = {AC[0] + P.PA[0] - Q.PA[0], AC[1] + P.PA[1] - Q.PA[1], AC[2] + P.PA[2] - Q.PA[2]};
           if (role == 2) {
             coop::rtab_poly(s.R, lane, PQ);
-          } else if (lane == 0) {
-            const double sum = P.p + Q.p, alpha = P.p * Q.p / sum;
-            coop::boys_rt(alpha * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]), s.R.L, boys, expt, s.R.base);
-            double f = 1.0;
-            for (int m = 0; m <= s.R.L; ++m) {
-              s.R.base[m] *= f;
-              f *= -2.0 * alpha;
-            }
-            s.S[0] = kTwoPiPow25 * P.kp * Q.kp * rsqrt(sum);
+          } else {
+            const double sum = P.p + Q.p, r = rsqrt(sum), alpha = P.p * Q.p * r * r;
+            coop::boys_base(alpha * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]), alpha, s.R.L, lane, boys, s.R.base);
+            if (lane == 0) s.S[0] = kTwoPiPow25 * P.kp * Q.kp * r;
           }
         }
       }
@@ -169,31 +170,60 @@ __device__ __forceinline__ void md_quartet(const MDShared& s, const PB& pb, int 
         coop::side_products(s.B, tid, nt, pref, false, s.R.S);
         if (first) coop::side_products(s.K, tid, nt, 1.0, true, s.R.S);
       });
-      // G[k][ab] (+)= sum_h E^{ab}_h R_{h+k}; neighbouring threads share ab
-      for (int x = tid; x < s.nab * nh; x += nt) {
-        const int ab = coop::fast_div(x, inv_nh), h = x - ab * nh;
-        const double* r = s.R.R + s.K.hlin[h];
-        double g = 0.0;
+      // G[k][ab] (+)= sum_h E^{ab}_h R_{h+k}: a thread takes up to four k of
+      // one ab, so that the products and their offsets are loaded once for
+      // four multiply-adds; neighbouring threads share ab
+      for (int x = tid; x < s.nab * nq; x += nt) {
+        const int ab = coop::fast_div(x, inv_nq), h = x - ab * nq;
+        const int h1 = min(h + nq, nh - 1), h2 = min(h + 2 * nq, nh - 1), h3 = min(h + 3 * nq, nh - 1);
+        const double *r0 = s.R.R + s.K.hlin[h], *r1 = s.R.R + s.K.hlin[h1], *r2 = s.R.R + s.K.hlin[h2],
+                     *r3 = s.R.R + s.K.hlin[h3];
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;
         const int k1 = s.B.start[ab + 1];
-        for (int k = s.B.start[ab]; k < k1; ++k) g = fma(s.B.prod[k], r[s.B.lin[k]], g);
-        double* o = s.G + h * s.gs + ab;
-        *o = first ? g : *o + g;
+#pragma unroll 2
+        for (int k = s.B.start[ab]; k < k1; ++k) {
+          const double f = s.B.prod[k];
+          const int o = s.B.lin[k];
+          g0 = fma(f, r0[o], g0);
+          g1 = fma(f, r1[o], g1);
+          g2 = fma(f, r2[o], g2);
+          g3 = fma(f, r3[o], g3);
+        }
+        double* o = s.G + ab;
+        auto put = [&](int k, double g) { o[k * s.gs] = first ? g : o[k * s.gs] + g; };
+        put(h, g0);
+        if (h + nq < nh) put(h1, g1);
+        if (h + 2 * nq < nh) put(h2, g2);
+        if (h + 3 * nq < nh) put(h3, g3);
       }
       first = false;
     }
     if (first) continue;  // every bra primitive screened out
     __syncthreads();
-    // out += sum_k E^{cd}_k G[k][ab]; neighbouring threads share cd
+    // out += sum_k E^{cd}_k G[k][ab], up to four ab of one cd per thread;
+    // neighbouring threads share cd
 #pragma unroll
-    for (int i = 0; i < ACC; ++i) {
+    for (int i = 0; i < ACC / 4; ++i) {
       const int x = tid + i * nt;
-      if (x < n) {
-        const int cd = coop::fast_div(x, inv_nab), ab = x - cd * s.nab;
+      if (x < s.ncd * s.na4) {
+        const int cd = coop::fast_div(x, s.inv_na4), ab = x - cd * s.na4;
         const double* g = s.G + ab;
-        double v = 0.0;
+        const int o1 = min(s.na4, s.nab - 1 - ab), o2 = min(2 * s.na4, s.nab - 1 - ab), o3 = min(3 * s.na4, s.nab - 1 - ab);
+        double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
         const int k1 = s.K.start[cd + 1];
-        for (int k = s.K.start[cd]; k < k1; ++k) v = fma(s.K.prod[k], g[s.K.h[k] * s.gs], v);
-        acc[i] += v;
+#pragma unroll 2
+        for (int k = s.K.start[cd]; k < k1; ++k) {
+          const double f = s.K.prod[k];
+          const double* r = g + s.K.h[k] * s.gs;
+          v0 = fma(f, r[0], v0);
+          v1 = fma(f, r[o1], v1);
+          v2 = fma(f, r[o2], v2);
+          v3 = fma(f, r[o3], v3);
+        }
+        acc[4 * i] += v0;
+        acc[4 * i + 1] += v1;
+        acc[4 * i + 2] += v2;
+        acc[4 * i + 3] += v3;
       }
     }
   }
@@ -202,15 +232,19 @@ __device__ __forceinline__ void md_quartet(const MDShared& s, const PB& pb, int 
 // acc scaled by f and the component scales into out[cd][ab].
 template <int ACC>
 __device__ __forceinline__ void md_store(const MDShared& s, const double (&acc)[ACC], double f) {
-  const int nt = blockDim.x, n = s.nab * s.ncd;
-  const float inv_nab = 1.0f / s.nab;
+  const int nt = blockDim.x;
   __syncthreads();  // G and R have been read
 #pragma unroll
-  for (int i = 0; i < ACC; ++i) {
+  for (int i = 0; i < ACC / 4; ++i) {
     const int x = threadIdx.x + i * nt;
-    if (x < n) {
-      const int cd = coop::fast_div(x, inv_nab), ab = x - cd * s.nab;
-      s.out[cd * s.os + ab] = acc[i] * f * s.B.scale[ab] * s.K.scale[cd];
+    if (x < s.ncd * s.na4) {
+      const int cd = coop::fast_div(x, s.inv_na4), ab0 = x - cd * s.na4;
+      const double fc = f * s.K.scale[cd];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int ab = ab0 + j * s.na4;
+        if (ab < s.nab) s.out[cd * s.os + ab] = acc[4 * i + j] * fc * s.B.scale[ab];
+      }
     }
   }
   __syncthreads();
@@ -220,10 +254,9 @@ __device__ __forceinline__ void md_store(const MDShared& s, const double (&acc)[
 // Schwarz bounds: shell pairs (prim_mode 0) or primitive pairs (prim_mode 1)
 // over persistent blocks, sqrt of the largest scaled diagonal element.
 template <int ACC>
-__global__ void __launch_bounds__(kMDThreads) schwarz_md_kernel(MDClass c, const PairInfo* __restrict__ pairs,
+__global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) schwarz_md_kernel(MDClass c, const PairInfo* __restrict__ pairs,
                                                                 const PrimPair* __restrict__ prims, int first,
                                                                 int count, const double* __restrict__ boys,
-                                                                const double* __restrict__ expt,
                                                                 double* __restrict__ out, int prim_mode) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   MDShared s;
@@ -236,7 +269,7 @@ __global__ void __launch_bounds__(kMDThreads) schwarz_md_kernel(MDClass c, const
     const double AB[3] = {owner.ABx, owner.ABy, owner.ABz}, AC[3] = {0.0, 0.0, 0.0};
     double acc[ACC];
     const PrimTable tab{prims + p0};
-    md_quartet<ACC>(s, tab, np, tab, np, AB, AB, AC, 0.0, boys, expt, acc);
+    md_quartet<ACC>(s, tab, np, tab, np, AB, AB, AC, 0.0, boys, acc);
     md_store<ACC>(s, acc, 1.0);
     double m = 0.0;
     for (int ij = threadIdx.x; ij < s.nab; ij += blockDim.x) m = fmax(m, s.out[ij * s.os + ij]);
@@ -253,10 +286,9 @@ __global__ void __launch_bounds__(kMDThreads) schwarz_md_kernel(MDClass c, const
 
 // One full scaled block (ab|cd) of bra pairs[0], ket pairs[1].
 template <int ACC>
-__global__ void __launch_bounds__(kMDThreads) quartet_md_kernel(MDClass c, const PairInfo* __restrict__ pairs,
+__global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) quartet_md_kernel(MDClass c, const PairInfo* __restrict__ pairs,
                                                                 const PrimPair* __restrict__ prims,
                                                                 const double* __restrict__ boys,
-                                                                const double* __restrict__ expt,
                                                                 double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   MDShared s;
@@ -266,7 +298,7 @@ __global__ void __launch_bounds__(kMDThreads) quartet_md_kernel(MDClass c, const
   const double AC[3] = {bra.Ax - ket.Ax, bra.Ay - ket.Ay, bra.Az - ket.Az};
   double acc[ACC];
   md_quartet<ACC>(s, PrimTable{prims + bra.pp_off}, bra.npp, PrimTable{prims + ket.pp_off}, ket.npp, AB, CD, AC, 0.0,
-                  boys, expt, acc);
+                  boys, acc);
   md_store<ACC>(s, acc, 1.0);
   for (int x = threadIdx.x; x < s.nab * s.ncd; x += blockDim.x) out[x] = s.out[(x % s.ncd) * s.os + x / s.ncd];
 }
@@ -278,25 +310,27 @@ __device__ __forceinline__ unsigned long long md_compound(unsigned long long i, 
 // Contracted block of (bra|ket) from the compact records.
 template <int ACC>
 __device__ __forceinline__ void md_quartet_rec(const MDShared& s, const PairInfo& bra, const PairInfo& ket,
-                                               const PrimRec64* __restrict__ rec, const float* __restrict__ pbound,
-                                               double eps, const double* __restrict__ boys,
-                                               const double* __restrict__ expt, double (&acc)[ACC]) {
+                                               unsigned slice, const PrimRec64* __restrict__ rec,
+                                               const float* __restrict__ pbound, double eps,
+                                               const double* __restrict__ boys,
+                                               double (&acc)[ACC]) {
   const double AB[3] = {bra.ABx, bra.ABy, bra.ABz}, CD[3] = {ket.ABx, ket.ABy, ket.ABz};
   const double AC[3] = {bra.Ax - ket.Ax, bra.Ay - ket.Ay, bra.Az - ket.Az};
-  const PrimRecs pb{rec, pbound, (size_t)bra.rec_off, (size_t)bra.rec_stride, AB};
-  const PrimRecs pk{rec, pbound, (size_t)ket.rec_off, (size_t)ket.rec_stride, CD};
-  md_quartet<ACC>(s, pb, bra.npp, pk, ket.npp, AB, CD, AC, eps, boys, expt, acc);
+  const PrimRange rb = prim_range(bra.rec_off, bra.rec_stride, bra.npp, slice, 0);
+  const PrimRange rk = prim_range(ket.rec_off, ket.rec_stride, ket.npp, slice, 16);
+  const PrimRecs pb{rec, pbound, (size_t)rb.off, (size_t)rb.stride, AB};
+  const PrimRecs pk{rec, pbound, (size_t)rk.off, (size_t)rk.stride, CD};
+  md_quartet<ACC>(s, pb, rb.count, pk, rk.count, AB, CD, AC, eps, boys, acc);
 }
 
 // Packed 8-fold tensor slots of the plan's quartets (the writer rules of
 // eri_packed_kernel: i >= j within a same-shell pair, IJ >= KL for a pair
 // with itself), over units of one ket of one warp task.
 template <int ACC>
-__global__ void __launch_bounds__(kMDThreads) eri_packed_md_kernel(
+__global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) eri_packed_md_kernel(
     MDClass c, const JKEntry* __restrict__ entries, const long long* __restrict__ prefix, int nentries,
     long long nwarps, const PairInfo* __restrict__ pairs, const double* __restrict__ pairQ, double thr,
-    const PrimRec64* __restrict__ rec, const float* __restrict__ pbound, const double* __restrict__ boys,
-    const double* __restrict__ expt, double* __restrict__ out) {
+    const PrimRec64* __restrict__ rec, const float* __restrict__ pbound, const double* __restrict__ boys, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   MDShared s;
   md_setup(c, smem_raw, s);
@@ -309,7 +343,7 @@ __global__ void __launch_bounds__(kMDThreads) eri_packed_md_kernel(
     if (kidx >= ent.k_hi || !(pairQ[kidx] * pairQ[ent.bra] > thr)) continue;
     const PairInfo bra = pairs[ent.bra], ket = pairs[kidx];
     double acc[ACC];
-    md_quartet_rec<ACC>(s, bra, ket, rec, pbound, 0.0, boys, expt, acc);
+    md_quartet_rec<ACC>(s, bra, ket, 0u, rec, pbound, 0.0, boys, acc);
     md_store<ACC>(s, acc, 1.0);
     const bool self = kidx == ent.bra;
     for (int x = threadIdx.x; x < s.nab * s.ncd; x += blockDim.x) {
@@ -325,42 +359,73 @@ __global__ void __launch_bounds__(kMDThreads) eri_packed_md_kernel(
   }
 }
 
-// Direct J/K (FP64) over a launch's work queue: persistent blocks take the
-// quartets one by one (or in short runs) and digest each as the fast kernels
-// do (jk_kernels.cuh): J'[a,b] += 4w sum D[c,d], J'[c,d] += 4w sum D[a,b],
+// Direct J/K (FP64) over a launch's work queue, for the classes with an f
+// shell and, of the others, the launches of few quartets in a class whose
+// generated code is too long to run cold (coop_launch in ctx.cu).  A unit of
+// work is one ket lane of one work-queue step; persistent blocks take units
+// in runs of `per` and digest each quartet as the fast kernels do
+// (jk_kernels.cuh): J'[a,b] += 4w sum D[c,d], J'[c,d] += 4w sum D[a,b],
 // K'[a,c] += 2w sum D[b,d] and the three other exchange blocks, w the
 // quartet's degeneracy weight.  In deterministic mode one block runs the
 // queue and one thread issues every atomic of a quartet, quartet after
-// quartet.
-template <int ACC>
-__global__ void __launch_bounds__(kMDThreads) jk_md_kernel(MDClass c, const JKLaunchArgs a) {
+// quartet.  BATCH: the queues of several molecules (RHF), as jk_batch_kernel.
+template <int ACC, bool BATCH>
+__global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) jk_md_kernel(MDClass c, const JKLaunchArgs args, int per) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   MDShared s;
   __shared__ long long s_unit;
   md_setup(c, smem_raw, s);
-  const int n = a.n, NS = a.nspin, tid = threadIdx.x, nt = blockDim.x;
+  JKLaunchArgs a = args;
+  const int NS = BATCH ? 1 : a.nspin, tid = threadIdx.x, nt = blockDim.x;
   const int na = c.na, nb = c.nb, nc = c.nc, nd = c.nd;
   double* Dcd = s.D;
   double* Dab = Dcd + nc * nd;
   double* Dk = Dab + na * nb;  // per spin: bd, ad, bc, ac
   const int nbd = nb * nd, nad = na * nd, nbc = nb * nc, nac = na * nc, nK = nbd + nad + nbc + nac;
-  const coop::UnitQueue uq = coop::unit_queue(a.chunk_start, a.nchunks, a.serial);
-  int e = 0;
   for (;;) {
     __syncthreads();
-    if (tid == 0) s_unit = (long long)atomicAdd(a.counter, (unsigned long long)uq.per);
+    if (tid == 0) s_unit = (long long)atomicAdd(args.counter, (unsigned long long)per);
     __syncthreads();
     const long long u0 = s_unit;
-    if (u0 >= uq.units) break;
-    for (long long u = u0; u < u0 + uq.per && u < uq.units; ++u) {
-      const long long w = uq.t0 + (u >> 5);
-      e = coop::entry_of(a.prefix, a.nentries, w, e);
+    if (u0 >= args.nchunks * 32) break;
+    // `per` divides 32: one step, lanes [lane0, lane0 + per) of its tasks
+    long long step = u0 >> 5;
+    const int lane0 = (int)(u0 & 31);
+    if (BATCH) {
+      int lo = 0, hi = args.njobs;  // last job whose first step is <= step
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(args.job_steps + mid) <= step) lo = mid; else hi = mid;
+      }
+      step -= __ldg(args.job_steps + lo);
+      const JKJob& jb = args.jobs[lo];
+      a.entries = jb.entries;
+      a.prefix = jb.prefix;
+      a.chunk_start = jb.chunk_start;
+      a.chunk_entry = jb.chunk_entry;
+      a.pairs = jb.pairs;
+      a.pairQ = jb.pairQ;
+      a.rec64 = jb.rec64;
+      a.pbound = jb.pbound;
+      a.Dtot = a.Dspin = jb.Dtot;
+      a.Jacc = jb.Jacc;
+      a.Kacc = jb.Kacc;
+      a.n = jb.n;
+      a.thr = jb.thr;
+      a.prim_eps = jb.prim_eps;
+    }
+    const int n = a.n;
+    const long long t0 = a.chunk_start[step], tasks = a.chunk_start[step + 1] - t0;
+    int e = a.chunk_entry[step];
+    for (long long u = 0; u < tasks * per; ++u) {
+      const long long w = t0 + u / per;
+      while (a.prefix[e + 1] <= w) ++e;
       const JKEntry ent = a.entries[e];
-      const int kidx = ent.k_lo + (int)(w - a.prefix[e]) * 32 + (int)(u & 31);
+      const int kidx = ent.k_lo + (int)(w - a.prefix[e]) * 32 + lane0 + (int)(u % per);
       if (kidx >= ent.k_hi || !(a.pairQ[kidx] * a.pairQ[ent.bra] > a.thr)) continue;
       const PairInfo bra = a.pairs[ent.bra], ket = a.pairs[kidx];
       double acc[ACC];
-      md_quartet_rec<ACC>(s, bra, ket, a.rec64, a.pbound, a.prim_eps, a.boys64, a.expt64, acc);
+      md_quartet_rec<ACC>(s, bra, ket, ent.slice, a.rec64, a.pbound, a.prim_eps, args.boys64, acc);
       double deg = 1.0;
       if (bra.same) deg *= 0.5;
       if (ket.same) deg *= 0.5;
@@ -451,9 +516,10 @@ int md_resident_blocks(const void* kern, int threads, size_t smem) {
   return sms * (per_sm > 0 ? per_sm : 1);
 }
 
-// the kernel instantiation of a class: 8 output elements per thread up to
-// 512 elements of the block (md_threads), 20 beyond
-#define HFG_MD_KERNEL(name, c) ((c).na * (c).nb * (c).nc * (c).nd <= 512 ? name<8> : name<kMDAcc>)
+// the kernel instantiation of a class: two items per thread up to 128 items
+// (md_threads), five beyond
+bool md_small(const MDClass& c) { return md_items(c) <= 128; }
+#define HFG_MD_KERNEL(name, c) (md_small(c) ? name<8> : name<kMDAcc>)
 
 }  // namespace
 
@@ -473,6 +539,11 @@ MDClass md_class(int la, int lb, int lc, int ld) {
   return c;
 }
 
+int md_blocks_per_sm(int la, int lb, int lc, int ld) {
+  const int nt = md_threads(md_class(la, lb, lc, ld));
+  return nt >= 512 ? 1 : (nt == 256 ? 2 : (nt == 128 ? 4 : 8));
+}
+
 bool md_class_ok(int la, int lb, int lc, int ld) {
   return la >= 0 && lb >= 0 && lc >= 0 && ld >= 0 && la <= kMDLMax && lb <= kMDLMax && lc <= kMDLMax &&
          ld <= kMDLMax;
@@ -488,7 +559,7 @@ cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimP
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c), grid = std::min(count, md_resident_blocks((const void*)kern, nt, smem));
-  kern<<<(unsigned)grid, nt, smem, st>>>(c, pairs, prims, first, count, boys, expt, out, prim_mode);
+  kern<<<(unsigned)grid, nt, smem, st>>>(c, pairs, prims, first, count, boys, out, prim_mode);
   return cudaGetLastError();
 }
 
@@ -500,7 +571,7 @@ cudaError_t launch_quartet_md(int la, int lb, int lc, int ld, const PairInfo* pa
   auto kern = HFG_MD_KERNEL(quartet_md_kernel, c);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<1, md_threads(c), smem, st>>>(c, pairs, prims, boys, expt, out);
+  kern<<<1, md_threads(c), smem, st>>>(c, pairs, prims, boys, out);
   return cudaGetLastError();
 }
 
@@ -518,8 +589,7 @@ cudaError_t launch_eri_packed_md(int la, int lb, int lc, int ld, const JKEntry* 
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c);
   const long long grid = std::min<long long>(nwarps * 32, md_resident_blocks((const void*)kern, nt, smem));
-  kern<<<(unsigned)grid, nt, smem, st>>>(c, entries, prefix, nentries, nwarps, pairs, pairQ, thr, rec, pbound, boys, expt,
-                                         out);
+  kern<<<(unsigned)grid, nt, smem, st>>>(c, entries, prefix, nentries, nwarps, pairs, pairQ, thr, rec, pbound, boys, out);
   return cudaGetLastError();
 }
 
@@ -528,12 +598,18 @@ cudaError_t launch_jk_md(int la, int lb, int lc, int ld, const JKLaunchArgs& a, 
   if (a.nchunks <= 0) return cudaSuccess;
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = md_smem(c, true);
-  auto kern = HFG_MD_KERNEL(jk_md_kernel, c);
+  const bool small = md_small(c);
+  auto kern = a.jobs ? (small ? jk_md_kernel<8, true> : jk_md_kernel<kMDAcc, true>)
+                     : (small ? jk_md_kernel<8, false> : jk_md_kernel<kMDAcc, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c);
-  const long long grid = a.serial ? 1 : std::min<long long>(a.nwarps * 32, md_resident_blocks((const void*)kern, nt, smem));
-  kern<<<(unsigned)grid, nt, smem, st>>>(c, a);
+  const long long units = a.nchunks * 32;
+  const long long grid = a.serial ? 1 : std::min<long long>(units, md_resident_blocks((const void*)kern, nt, smem));
+  // short runs while there are units to spare for every block
+  int per = a.serial ? 32 : 1;
+  while (per < 32 && units > 2LL * per * grid * 16) per *= 2;
+  kern<<<(unsigned)grid, nt, smem, st>>>(c, a, per);
   return cudaGetLastError();
 }
 

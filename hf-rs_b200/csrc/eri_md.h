@@ -29,6 +29,11 @@ cudaError_t launch_eri_packed_md(int la, int lb, int lc, int ld, const JKEntry* 
                                  const double* expt, double* out, cudaStream_t st);
 // FP64 J/K over the launch's work queue (a.serial: one block, deterministic)
 cudaError_t launch_jk_md(int la, int lb, int lc, int ld, const JKLaunchArgs& a, cudaStream_t st);
+// Blocks of the J/K engine that an SM holds, about (by the class's block size)
+int md_blocks_per_sm(int la, int lb, int lc, int ld);
+// Whether the class's gradient kernel splits a quartet's primitive quartets
+// over lanes by itself (the others take sliced entries)
+bool eri_gradient_splits(int la, int lb, int lc, int ld);
 // Nuclear derivatives of the two-electron energy over the launch's work
 // queue (grad.cu; densities a.Dtot, a.Dspin; shells up to d): adds into
 // grad[natom][3]

@@ -256,14 +256,21 @@ size_t coop_smem(const MDClass& c) {
 
 // products of a side listed by Hermite index
 __device__ void list_by_herm(const coop::Side& s, int* start, unsigned short* list) {
-  for (int h = threadIdx.x; h <= s.nh; h += blockDim.x) {
+  // a warp per Hermite index: 32 products a step, placed by ballot
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int h = warp; h < s.nh; h += nw) {
     int n = 0;
-    for (int k = 0; k < s.nnz; ++k) n += s.h[k] < h;
-    start[h] = n;
-    if (h < s.nh)
-      for (int k = 0; k < s.nnz; ++k)
-        if (s.h[k] == h) list[n++] = (unsigned short)k;
+    for (int k0 = 0; k0 < s.nnz; k0 += 32)
+      n += __popc(__ballot_sync(0xffffffffu, k0 + lane < s.nnz && s.h[k0 + lane] < h));
+    if (lane == 0) start[h] = n;
+    for (int k0 = 0; k0 < s.nnz; k0 += 32) {
+      const bool mine = k0 + lane < s.nnz && s.h[k0 + lane] == h;
+      const unsigned b = __ballot_sync(0xffffffffu, mine);
+      if (mine) list[n + __popc(b & ((1u << lane) - 1u))] = (unsigned short)(k0 + lane);
+      n += __popc(b);
+    }
   }
+  if (threadIdx.x == 0) start[s.nh] = s.nnz;
 }
 
 __global__ void __launch_bounds__(kCoopThreads) grad_coop_kernel(MDClass c, const GradArgs a) {
@@ -325,11 +332,13 @@ __global__ void __launch_bounds__(kCoopThreads) grad_coop_kernel(MDClass c, cons
       for (int k = 0; k < 9; ++k) acc[k] = 0.0;
       const double AB[3] = {bra.ABx, bra.ABy, bra.ABz}, CD[3] = {ket.ABx, ket.ABy, ket.ABz};
       const double AC[3] = {bra.Ax - ket.Ax, bra.Ay - ket.Ay, bra.Az - ket.Az};
-      for (int ib = 0; ib < bra.npp; ++ib) {
-        const PrimRec64 rb = a.rec[bra.rec_off + (size_t)ib * bra.rec_stride];
+      const PrimRange pb = prim_range(bra.rec_off, bra.rec_stride, bra.npp, ent.slice, 0);
+      const PrimRange pk = prim_range(ket.rec_off, ket.rec_stride, ket.npp, ent.slice, 16);
+      for (int ib = 0; ib < pb.count; ++ib) {
+        const PrimRec64 rb = a.rec[pb.off + (size_t)ib * pb.stride];
         bool fresh = true;  // this bra primitive's tables are not made yet
-        for (int ik = 0; ik < ket.npp; ++ik) {
-          const PrimRec64 rk = a.rec[ket.rec_off + (size_t)ik * ket.rec_stride];
+        for (int ik = 0; ik < pk.count; ++ik) {
+          const PrimRec64 rk = a.rec[pk.off + (size_t)ik * pk.stride];
           const double kpq = rb.kp * rk.kp;
           if (fabs(kpq) < kPrimFloor) continue;  // (the same for every thread)
           __syncthreads();
@@ -344,15 +353,10 @@ __global__ void __launch_bounds__(kCoopThreads) grad_coop_kernel(MDClass c, cons
             const double PQ[3] = {AC[0] + PA[0] - QC[0], AC[1] + PA[1] - QC[1], AC[2] + PA[2] - QC[2]};
             if (warp == 2) {
               coop::rtab_poly(R, lane, PQ);
-            } else if (lane == 0) {
-              const double sum = rb.p + rk.p, alpha = rb.p * rk.p / sum;
-              coop::boys_rt(alpha * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]), R.L, a.boys, a.expt, R.base);
-              double f = 1.0;
-              for (int m = 0; m <= R.L; ++m) {
-                R.base[m] *= f;
-                f *= -2.0 * alpha;
-              }
-              S[3] = kTwoPiPow25 * kpq * rsqrt(sum);
+            } else {
+              const double sum = rb.p + rk.p, r = rsqrt(sum), alpha = rb.p * rk.p * r * r;
+              coop::boys_base(alpha * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]), alpha, R.L, lane, a.boys, R.base);
+              if (lane == 0) S[3] = kTwoPiPow25 * kpq * r;
             }
           }
           __syncthreads();
@@ -470,6 +474,10 @@ cudaError_t launch_lane(const GradArgs& a, long long ntasks, cudaStream_t st) {
 }
 
 }  // namespace
+
+bool eri_gradient_splits(int la, int lb, int lc, int ld) {
+  return la + lb + lc + ld <= 4 && !(la == 2 && lb == 1 && lc == 1 && ld == 0);
+}
 
 cudaError_t launch_eri_gradient(int la, int lb, int lc, int ld, const JKLaunchArgs& j, const int* ao_atom, int natom,
                                 double* grad, cudaStream_t st) {

@@ -37,6 +37,7 @@ struct Launch {
   int la, lb, lc, ld;
   cudaStream_t st = nullptr;  // stream of the entries/prefix allocations
   bool fp32;
+  bool coop = false;  // runs on the block-per-quartet engine (eri_md.cu)
   double quartets = 0, prims = 0;  // shell quartets and primitive quartets (after screening) of this launch
   std::vector<JKEntry> entries;
   std::vector<long long> prefix;
@@ -48,10 +49,23 @@ struct Launch {
   std::vector<double> cost_prefix;  // nominal cost of steps [0, c) (nchunks + 1)
 };
 
+// What a plan's entries are sliced for: one J/K build, consumers that need
+// every quartet whole (the packed tensor), a batched build (many molecules
+// fill the GPU: coarser slices), the gradient (whose lane kernel splits the
+// primitive quartets by itself: slices for the other classes only).
+enum PlanUse { kPlanJK = 0, kPlanWhole = 1, kPlanBatch = 2, kPlanGrad = 3 };
+
+// side streams on which a J/K build's class launches (and the other sets of
+// independent launches) run next to the context stream: a small molecule's
+// 21 launches each use a few SMs (one water 250 us on 4 streams, 207 on 8)
+constexpr int kJKSideStreams = 7;
+
 struct Plan {
   std::vector<Launch> launches;
   hfg_jk_stats stats{};  // nominal counts until `counted`
   double thr = 0.0, prim_eps = 0.0;
+  bool sliced = false;   // some entries are slices of quartets
+  int streams = 1 + kJKSideStreams;  // concurrent launches of a build
   bool counted = false;  // exact shell/primitive-quartet counts made (on the first stats request)
 };
 
@@ -99,9 +113,6 @@ template <typename T> struct DevBuf {
 }  // namespace hfg
 
 namespace hfg {
-// side streams on which a J/K build's class launches run next to the
-// context stream
-constexpr int kJKSideStreams = 3;
 // Collects the RHF J/K builds of several contexts into batched builds
 // (server.cu); a context with one set routes its builds through it.
 struct JKBatcher;
@@ -115,20 +126,24 @@ struct hfg_ctx {
   cudaStream_t side[hfg::kJKSideStreams] = {};
   hfg::JKBatcher* batcher = nullptr;  // RHF builds go through this batcher when set
   cudaEvent_t ev_fork = nullptr, ev_join[hfg::kJKSideStreams] = {};
+  cudaError_t ensure_fork() {
+    return ev_fork ? cudaSuccess : cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
+  }
   cudaError_t ensure_side_streams() {
-    if (ev_fork) return cudaSuccess;
-    // the side streams take the context stream's priority
-    int prio = 0;
-    if (stream && cudaStreamGetPriority(stream, &prio) != cudaSuccess) prio = 0;
-    for (auto& x : side) {
-      const cudaError_t e = cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio);
-      if (e != cudaSuccess) return e;
+    if (!ev_join[hfg::kJKSideStreams - 1]) {
+      // the side streams take the context stream's priority
+      int prio = 0;
+      if (stream && cudaStreamGetPriority(stream, &prio) != cudaSuccess) prio = 0;
+      for (auto& x : side) {
+        const cudaError_t e = x ? cudaSuccess : cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio);
+        if (e != cudaSuccess) return e;
+      }
+      for (auto& x : ev_join) {
+        const cudaError_t e = x ? cudaSuccess : cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+      }
     }
-    for (auto& x : ev_join) {
-      const cudaError_t e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
+    return ensure_fork();
   }
   std::mutex mu;
   std::string err;
@@ -169,7 +184,10 @@ struct hfg_ctx {
   hfg::DevBuf<float> d_D32;  // FP32 copies of a build's densities (3 n^2)
 
   // launch plans by (Schwarz, FP32 and primitive thresholds, precision, tile)
-  std::map<std::tuple<double, double, double, int, int>, std::unique_ptr<hfg::Plan>> plans;
+  // and, where the J/K plan slices quartets, those sliced otherwise for the
+  // other uses (PlanUse - 1)
+  using PlanMap = std::map<std::tuple<double, double, double, int, int>, std::unique_ptr<hfg::Plan>>;
+  PlanMap plans, other_plans[3];
   hfg_jk_stats last{};
 
   ~hfg_ctx();

@@ -56,11 +56,31 @@ struct KetSoA {
   const int2* nn;     // npp, same
 };
 
-// Work entry of one J/K launch: bra pair and the range of ket pairs
-// [k_lo, k_hi) (global pair indices, kets of one pair class).
+// Work entry of one launch: bra pair and the range of ket pairs [k_lo, k_hi)
+// (global pair indices, kets of one pair class).  `slice` is 0 for whole
+// quartets; else the entry covers one slice of the primitive quartets, bra
+// primitive pairs sb, sb + nb, ... and ket ones sk, sk + nk, ..., with sb,
+// nb, sk, nk in its bytes from the lowest (J and K are linear in the
+// integrals, so slices are digested one by one like quartets).
 struct JKEntry {
-  int bra, k_lo, k_hi, pad;
+  int bra, k_lo, k_hi;
+  unsigned slice;
 };
+
+// The primitive pairs of one side of an entry: first record, record stride
+// and count, from the pair's own and the side's slice bytes (s, of).
+struct PrimRange {
+  int off, stride, count;
+};
+__host__ __device__ __forceinline__ PrimRange prim_range(int off, int stride, int count, unsigned slice, int shift) {
+  if (slice) {
+    const int s = (slice >> shift) & 255, of = (slice >> (shift + 8)) & 255;
+    off += s * stride;
+    stride *= of;
+    count = (count - s + of - 1) / of;
+  }
+  return PrimRange{off, stride, count};
+}
 
 // One molecule of a batched J/K launch: its launch's work queue and the
 // buffers of its context (RHF: the total density is the spin density).

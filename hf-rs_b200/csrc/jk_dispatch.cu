@@ -7,9 +7,9 @@
 
 namespace hfg {
 
-cudaError_t launch_jk(int la, int lb, int lc, int ld, bool fp32, const JKLaunchArgs& a, cudaStream_t st) {
+cudaError_t launch_jk(int la, int lb, int lc, int ld, bool fp32, bool coop, const JKLaunchArgs& a, cudaStream_t st) {
   // classes with an f shell: the generic engine, FP64 only
-  if (la > kLMax || lb > kLMax || lc > kLMax || ld > kLMax)
+  if (coop || la > kLMax || lb > kLMax || lc > kLMax || ld > kLMax)
     return fp32 ? cudaErrorInvalidValue : launch_jk_md(la, lb, lc, ld, a, st);
 #define HFG_CASE(A, B, C, D) \
   if (la == A && lb == B && lc == C && ld == D) return launch_jk_##A##B##C##D(a, fp32, st);
@@ -38,7 +38,9 @@ cudaError_t launch_jk(int la, int lb, int lc, int ld, bool fp32, const JKLaunchA
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_jk_batch(int la, int lb, int lc, int ld, bool fp32, const JKLaunchArgs& a, cudaStream_t st) {
+cudaError_t launch_jk_batch(int la, int lb, int lc, int ld, bool fp32, bool coop, const JKLaunchArgs& a,
+                            cudaStream_t st) {
+  if (coop) return fp32 ? cudaErrorInvalidValue : launch_jk_md(la, lb, lc, ld, a, st);
   if (la > kLMax || lb > kLMax || lc > kLMax || ld > kLMax) return cudaErrorInvalidValue;
 #define HFG_CASE(A, B, C, D) \
   if (la == A && lb == B && lc == C && ld == D) return launch_jkb_##A##B##C##D(a, fp32, st);

@@ -32,9 +32,12 @@ HFG_DECL(2, 2, 2, 1)
 HFG_DECL(2, 2, 2, 2)
 #undef HFG_DECL
 
-cudaError_t launch_jk(int la, int lb, int lc, int ld, bool fp32, const JKLaunchArgs& a, cudaStream_t st);
+// coop: on the block-per-quartet engine (FP64; classes with an f shell always
+// run there)
+cudaError_t launch_jk(int la, int lb, int lc, int ld, bool fp32, bool coop, const JKLaunchArgs& a, cudaStream_t st);
 // The same over several molecules (a.jobs, a.job_steps, a.njobs; RHF).
-cudaError_t launch_jk_batch(int la, int lb, int lc, int ld, bool fp32, const JKLaunchArgs& a, cudaStream_t st);
+cudaError_t launch_jk_batch(int la, int lb, int lc, int ld, bool fp32, bool coop, const JKLaunchArgs& a,
+                            cudaStream_t st);
 cudaError_t launch_schwarz(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,
                            const double* boys, const double* expt, double* out, int prim_mode, cudaStream_t st);
 // out[0] += evaluated primitive quartets, out[1] += evaluated shell quartets

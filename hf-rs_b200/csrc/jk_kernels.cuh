@@ -304,11 +304,16 @@ __device__ __forceinline__ void jk_step(const JKLaunchArgs& a, long long c, int 
           const T ACx = (T)(bra.Ax - ket.Ax), ACy = (T)(bra.Ay - ket.Ay), ACz = (T)(bra.Az - ket.Az);
           const T bABx = (T)bra.ABx, bABy = (T)bra.ABy, bABz = (T)bra.ABz;
           const T kABx = (T)ket.ABx, kABy = (T)ket.ABy, kABz = (T)ket.ABz;
-          const Rec* __restrict__ br = RecOf<T>::get(a) + bra.rec_off;
-          const Rec* __restrict__ kr = RecOf<T>::get(a) + ket.rec_off;
-          const float* __restrict__ bb = a.pbound + bra.rec_off;
-          const float* __restrict__ kb = a.pbound + ket.rec_off;
-          const int nb = bra.npp, nk = ket.npp, bs = bra.rec_stride, ks = ket.rec_stride;
+          // (only FP64 launches are sliced: the test costs the light FP32
+          // classes 1%)
+          const unsigned slice = sizeof(T) == 8 ? ent.slice : 0u;
+          const PrimRange rb = prim_range(bra.rec_off, bra.rec_stride, bra.npp, slice, 0);
+          const PrimRange rk = prim_range(ket.rec_off, ket.rec_stride, ket.npp, slice, 16);
+          const Rec* __restrict__ br = RecOf<T>::get(a) + rb.off;
+          const Rec* __restrict__ kr = RecOf<T>::get(a) + rk.off;
+          const float* __restrict__ bb = a.pbound + rb.off;
+          const float* __restrict__ kb = a.pbound + rk.off;
+          const int nb = rb.count, nk = rk.count, bs = rb.stride, ks = rk.stride;
           // screening products in FP32 (bounds are stored as floats; count_kernel
           // evaluates the same products)
           const float eps = (float)a.prim_eps;

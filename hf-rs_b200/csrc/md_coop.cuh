@@ -273,45 +273,34 @@ __device__ __forceinline__ void side_products(const Side& s, int tid, int nt, do
   }
 }
 
-// F_0..F_L at T for a run-time L <= 16: the device's Boys scheme (boys.cuh)
-// read from the global grid table (kBoysCols columns per row).
-__device__ inline void boys_rt(double t, int L, const double* __restrict__ table, const double* __restrict__ expt,
-                               double* F) {
+// base[m] = (-2 alpha)^m F_m(T), m <= L <= 16, by one warp, order m on lane m:
+// each order by its own Taylor row of the global grid table (kBoysCols
+// columns per row; boys.cuh's expansion without its downward recursion, whose
+// divisions made a chain through every order), the asymptotic form beyond
+// the grid by upward recursion on each lane.
+__device__ __forceinline__ void boys_base(double t, double alpha, int L, int lane, const double* __restrict__ table,
+                                          double* base) {
+  if (lane > L) return;
+  double f;
   if (t > kBoysTMax) {
-    const double r = rsqrt(t);
-    double f = kHalfSqrtPi * r;
-    F[0] = f;
-    const double inv2t = 0.5 * r * r, e = exp(-t);
-    for (int m = 1; m <= L; ++m) {
-      f = ((2 * m - 1) * f - e) * inv2t;
-      F[m] = f;
-    }
-    return;
+    const double r = rsqrt(t), inv2t = 0.5 * r * r, e = exp(-t);
+    f = kHalfSqrtPi * r;
+    for (int m = 1; m <= lane; ++m) f = ((2 * m - 1) * f - e) * inv2t;
+  } else {
+    const int idx = min(max(__double2int_rn(t * 20.0), 0), kBoysSmemRows - 1);
+    const double x = idx * kBoysStep - t;
+    const double* row = table + (size_t)idx * kBoysCols + lane;
+    f = __ldg(row + 7) * (1.0 / 5040.0);
+    f = fma(f, x, __ldg(row + 6) * (1.0 / 720.0));
+    f = fma(f, x, __ldg(row + 5) * (1.0 / 120.0));
+    f = fma(f, x, __ldg(row + 4) * (1.0 / 24.0));
+    f = fma(f, x, __ldg(row + 3) * (1.0 / 6.0));
+    f = fma(f, x, __ldg(row + 2) * 0.5);
+    f = fma(f, x, __ldg(row + 1));
+    f = fma(f, x, __ldg(row));
   }
-  const int idx = min(max(__double2int_rn(t * 20.0), 0), kBoysSmemRows - 1);
-  const double x = idx * kBoysStep - t;
-  const double* row = table + (size_t)idx * kBoysCols + L;
-  double acc = row[7] * (1.0 / 5040.0);
-  acc = fma(acc, x, row[6] * (1.0 / 720.0));
-  acc = fma(acc, x, row[5] * (1.0 / 120.0));
-  acc = fma(acc, x, row[4] * (1.0 / 24.0));
-  acc = fma(acc, x, row[3] * (1.0 / 6.0));
-  acc = fma(acc, x, row[2] * 0.5);
-  acc = fma(acc, x, row[1]);
-  double f = fma(acc, x, row[0]);
-  F[L] = f;
-  double ex = fma(x, 1.0 / 5040.0, 1.0 / 720.0);
-  ex = fma(ex, x, 1.0 / 120.0);
-  ex = fma(ex, x, 1.0 / 24.0);
-  ex = fma(ex, x, 1.0 / 6.0);
-  ex = fma(ex, x, 0.5);
-  ex = fma(ex, x, 1.0);
-  ex = fma(ex, x, 1.0);
-  const double e = expt[idx] * ex, t2 = 2.0 * t;
-  for (int m = L - 1; m >= 0; --m) {
-    f = fma(t2, f, e) / (2 * m + 1);
-    F[m] = f;
-  }
+  for (int m = 0; m < lane; ++m) f *= -2.0 * alpha;
+  base[lane] = f;
 }
 
 // The R tables of one quartet: base orders, one-axis polynomials, the two

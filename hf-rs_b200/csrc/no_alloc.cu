@@ -98,9 +98,16 @@ extern "C" int hfg_jk_device_noalloc(hfg_ctx* ctx, const hfg_jk_opts* opts, int 
   if (256 + (size_t)(1 + nspin) * nn * sizeof(double) > kScratchBytes)
     return hfg::set_error(ctx, HFG_ERR_INVALID_INPUT, too_big);
   std::lock_guard<std::mutex> lk(ctx->mu);
-  auto it = ctx->plans.find(std::make_tuple(o.schwarz_threshold, o.precision == HFG_MIXED ? o.mixed_threshold : 0.0,
-                                            o.prim_threshold, o.precision, o.tile > 0 ? o.tile : 64));
-  if (it == ctx->plans.end())
+  const auto key = std::make_tuple(o.schwarz_threshold, o.precision == HFG_MIXED ? o.mixed_threshold : 0.0,
+                                   o.prim_threshold, o.precision, o.tile > 0 ? o.tile : 64);
+  auto it = ctx->plans.find(key);
+  bool found = it != ctx->plans.end();
+  for (auto& m : ctx->other_plans) {
+    if (found) break;
+    it = m.find(key);
+    found = it != m.end();
+  }
+  if (!found)
     return hfg::set_error(ctx, HFG_ERR_INVALID_INPUT,
                           "hfg_jk_device_noalloc: no launch plan for these options on this context; call hfg_jk or "
                           "hfg_jk_device once with them first (that call allocates the plan)");
@@ -165,7 +172,7 @@ extern "C" int hfg_jk_device_noalloc(hfg_ctx* ctx, const hfg_jk_opts* opts, int 
     a.nchunks = L.nchunks;
     a.nentries = (int)L.prefix[0];
     a.nwarps = L.prefix[1];
-    rc = hfg::cuda_check(ctx, hfg::launch_jk(L.la, L.lb, L.lc, L.ld, L.fp32, a, ctx->stream), "J/K launch");
+    rc = hfg::cuda_check(ctx, hfg::launch_jk(L.la, L.lb, L.lc, L.ld, L.fp32, L.coop, a, ctx->stream), "J/K launch");
     if (rc != HFG_OK) return rc;
   }
   const int blk = 256;

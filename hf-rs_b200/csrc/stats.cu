@@ -27,20 +27,23 @@ __global__ void count_kernel(const JKEntry* __restrict__ entries, const long lon
   const int k = e.k_lo + (int)(warp - prefix[lo]) * 32 + lane;
   unsigned long long c = 0, quartets = 0;
   if (k < e.k_hi && pairQ[k] * pairQ[e.bra] > thr) {
-    quartets = 1;
+    // a sliced quartet is counted with its first slice
+    quartets = (e.slice & 0xff00ffu) == 0 ? 1 : 0;
     const PairInfo b = pairs[e.bra], q = pairs[k];
+    const PrimRange rb = prim_range(b.rec_off, b.rec_stride, b.npp, e.slice, 0);
+    const PrimRange rk = prim_range(q.rec_off, q.rec_stride, q.npp, e.slice, 16);
     // the kernels' loop: ket primitive pairs surviving against the largest bra
     // one, then bra primitive pairs while the product stays above eps
     // (FP32 products, as in the kernels)
     const float feps = (float)eps;
-    const float bmax = pbound[b.rec_off];
-    for (int ik = 0; ik < q.npp; ++ik) {
-      const float qb = pbound[q.rec_off + (size_t)ik * q.rec_stride];
+    const float bmax = pbound[rb.off];
+    for (int ik = 0; ik < rk.count; ++ik) {
+      const float qb = pbound[rk.off + (size_t)ik * rk.stride];
       if (qb * bmax < feps) break;
-      int l = 0, h = b.npp;  // bounds sorted descending
+      int l = 0, h = rb.count;  // bounds sorted descending
       while (l < h) {
         const int m = (l + h) >> 1;
-        if (pbound[b.rec_off + (size_t)m * b.rec_stride] * qb >= feps) l = m + 1; else h = m;
+        if (pbound[rb.off + (size_t)m * rb.stride] * qb >= feps) l = m + 1; else h = m;
       }
       c += (unsigned long long)l;
     }
