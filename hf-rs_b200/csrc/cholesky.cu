@@ -12,11 +12,9 @@
 // (packed 8-fold, from the J/K engine's integrals for quartets with
 // Q_ab Q_cd > 1e-15, the column filter hf-rs uses), which bounds the
 // system size to n_p (n_p + 1) / 2 doubles of device memory; hf-rs instead
-// evaluates the pivots' columns on the fly.  Each step: the residual
-// diagonal comes back to the host (the pivot rule must match exactly), the
-// pivot column is gathered from V, the previous vectors' projection is
-// removed with one DGEMV, and the diagonal is updated and checked on the
-// device.
+// evaluates the pivots' columns on the fly.  All steps run in one kernel
+// (chol_kernel): each block keeps a range of columns, and a step is one
+// barrier over the grid.
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
@@ -39,22 +37,180 @@ __global__ void chol_diag_kernel(const double* __restrict__ V, long long np, dou
     d[k] = V[packed(k, k)];
 }
 
-__global__ void chol_column_kernel(const double* __restrict__ V, long long np, long long pivot, double* __restrict__ c) {
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < np; k += (long long)gridDim.x * blockDim.x)
-    c[k] = V[packed(k, pivot)];
+// The decomposition itself: one cooperative launch, each block owning the
+// columns [b per, (b + 1) per).  A step:
+//
+//   1. the block's largest residual diagonal goes to bmax; grid barrier;
+//   2. every block finds the largest M of all, and the pivot: the first
+//      column with d >= M - 1e-12 |M|, which lies in the first block range
+//      whose own maximum reaches that bound (hf-rs's tie rule);
+//   3. for its own columns, row = (V[:, pivot] - sum_K L_K L_K[pivot]) / root
+//      and diag -= row^2, with the check and clamp of src/cholesky.rs:172-178.
+//
+// A step costs the barrier and the pass over the vectors so far (8 rank n_p
+// bytes, from L2); the earlier form, three launches, a copy of the diagonal
+// and a host scan per pivot, took 52 us per pivot at n_p = 2,850.
+// The vectors' sum runs over 8 interleaved parts (one per warp) added in a
+// fixed order, the same for every column, so equivalent pairs of a symmetric
+// molecule keep equal residuals.
+constexpr int kCholThreads = 256, kCholCols = 32, kCholPiv = 4096;
+constexpr unsigned long long kCholWaitNs = 2000000000ull;
+
+struct CholState {
+  unsigned arrived;     // blocks that have reached the barrier, over all steps
+  int bad;              // a residual diagonal fell below -1e-10 scale
+  int status;           // 0 running, 1 done, 2 budget, 3 a bounded wait ran out
+  long long rank;
+  double residual;
+};
+
+struct CholArgs {
+  const double* V;
+  double* L;        // [cap][np]
+  double* diag;     // [2][np], step r reads half r & 1 and writes the other
+  double* bmax;     // [2][blocks], likewise
+  CholState* st;
+  long long* piv;   // [cap]
+  long long np, cap, per;
+  double threshold, scale, budget;
+};
+
+__device__ __forceinline__ unsigned long long chol_clock() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
 }
 
-// row = column / root with row[pivot] = root; diag -= row^2, with the check
-// and clamp of src/cholesky.rs:172-178 (bad[0] set on a residual below
-// -1e-10 scale)
-__global__ void chol_update_kernel(double* __restrict__ row, long long np, long long pivot, double root, double scale,
-                                   double* __restrict__ diag, int* __restrict__ bad) {
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < np; k += (long long)gridDim.x * blockDim.x) {
-    const double r = k == pivot ? root : row[k] / root;
-    row[k] = r;
-    const double d = diag[k] - r * r;
-    if (d < -1e-10 * scale) *bad = 1;
-    diag[k] = fmax(d, 0.0);
+// Barrier over the grid (all blocks resident): false when it gave up, after
+// 2 s or because another block did.
+__device__ __forceinline__ bool chol_barrier(CholState* st, unsigned target, int* ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&st->arrived, 1u);
+    unsigned long long t0 = 0;
+    int good = 1;
+    for (unsigned i = 1; *(volatile unsigned*)&st->arrived < target; ++i) {
+      if ((i & 255u) != 0) continue;  // (a read of the clock costs more than most waits)
+      const unsigned long long now = chol_clock();
+      if (t0 == 0) t0 = now;
+      if (*(volatile int*)&st->status == 3 || now - t0 > kCholWaitNs) {
+        atomicExch(&st->status, 3);
+        good = 0;
+        break;
+      }
+    }
+    __threadfence();
+    *ok = good;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+__device__ __forceinline__ double block_max(double v, double* red) {
+  for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+  for (int k = 1; k < kCholThreads / 32; ++k) v = fmax(v, red[k]);
+  return v;
+}
+__device__ __forceinline__ long long block_min(long long v, long long* red) {
+  for (int off = 16; off > 0; off >>= 1) {
+    const long long o = __shfl_xor_sync(0xffffffffu, v, off);
+    v = o < v ? o : v;
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+  for (int k = 1; k < kCholThreads / 32; ++k) v = red[k] < v ? red[k] : v;
+  return v;
+}
+
+__global__ void __launch_bounds__(kCholThreads) chol_kernel(const CholArgs a) {
+  __shared__ double redd[kCholThreads / 32];
+  __shared__ long long redl[kCholThreads / 32];
+  __shared__ double part[kCholThreads / 32][kCholCols];
+  __shared__ double lp[kCholPiv];
+  __shared__ int ok;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, G = gridDim.x;
+  const long long none = 0x7fffffffffffffffLL;
+  const long long c0 = blockIdx.x * a.per, c1 = min(a.np, c0 + a.per);
+  unsigned target = 0;
+  for (long long rank = 0;; ++rank) {
+    const double* diag = a.diag + (rank & 1) * a.np;
+    double* next = a.diag + ((rank + 1) & 1) * a.np;
+    double m = -INFINITY;
+    for (long long k = c0 + tid; k < c1; k += kCholThreads) m = fmax(m, __ldcg(diag + k));
+    m = block_max(m, redd);
+    double* bm = a.bmax + (rank & 1) * G;
+    if (tid == 0) __stcg(bm + blockIdx.x, m);
+    target += G;
+    if (!chol_barrier(a.st, target, &ok)) return;
+    if (*(volatile int*)&a.st->bad) {
+      if (blockIdx.x == 0 && tid == 0) a.st->rank = rank;
+      return;
+    }
+    m = -INFINITY;
+    for (int b = tid; b < G; b += kCholThreads) m = fmax(m, __ldcg(bm + b));
+    const double largest = block_max(m, redd), bound = largest - 1e-12 * fabs(largest);
+    long long first = none;
+    for (int b = tid; b < G; b += kCholThreads)
+      if (__ldcg(bm + b) >= bound && b < first) first = b;
+    const long long owner = block_min(first, redl);
+    first = none;
+    const long long o1 = min(a.np, (owner + 1) * a.per);
+    for (long long k = owner * a.per + tid; k < o1; k += kCholThreads)
+      if (__ldcg(diag + k) >= bound) {
+        first = k;
+        break;
+      }
+    const long long pivot = block_min(first, redl);
+    if (pivot == none) {  // no finite diagonal is left
+      if (blockIdx.x == 0 && tid == 0) a.st->bad = 1;
+      return;
+    }
+    const double maximum = __ldcg(diag + pivot);
+    const bool done = maximum <= a.threshold || rank == a.np;
+    if (done || 8.0 * (double)a.np * (double)(rank + 2) > a.budget || rank >= a.cap) {
+      if (blockIdx.x == 0 && tid == 0) {
+        a.st->rank = rank;
+        a.st->residual = fmax(maximum, 0.0);
+        a.st->status = done ? 1 : 2;
+      }
+      return;
+    }
+    if (blockIdx.x == 0 && tid == 0) a.piv[rank] = pivot;
+    const double root = sqrt(maximum);
+    for (long long k = tid; k < rank && k < kCholPiv; k += kCholThreads) lp[k] = __ldcg(a.L + k * a.np + pivot);
+    __syncthreads();
+    double* row = a.L + rank * a.np;
+    for (long long t = c0; t < c1; t += kCholCols) {
+      const long long k = t + lane;
+      double s = 0.0;
+      if (k < c1) {
+        const double* l = a.L + k;
+        const long long r1 = rank < kCholPiv ? rank : kCholPiv;
+        long long K = warp;
+#pragma unroll 4
+        for (; K < r1; K += kCholThreads / 32) s = fma(lp[K], l[K * a.np], s);
+        for (; K < rank; K += kCholThreads / 32) s = fma(__ldcg(a.L + K * a.np + pivot), l[K * a.np], s);
+      }
+      part[warp][lane] = s;
+      __syncthreads();
+      if (warp == 0 && k < c1) {
+        double v = a.V[packed(k, pivot)];
+        for (int w = 0; w < kCholThreads / 32; ++w) v -= part[w][lane];
+        const double r = k == pivot ? root : v / root;
+        __stcg(row + k, r);
+        const double d = __ldcg(diag + k) - r * r;
+        if (d < -1e-10 * a.scale) a.st->bad = 1;
+        __stcg(next + k, fmax(d, 0.0));
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -79,21 +235,17 @@ extern "C" int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, h
     rc = cuda_check(ctx, (call), #call); \
     if (rc != HFG_OK) return rc;         \
   } while (0)
-  DevBuf<double> V, diag, col;
-  DevBuf<int> bad;
+  DevBuf<double> V, diag;
   if (V.alloc(vlen) != cudaSuccess) {
     cudaGetLastError();
     return set_error(ctx, HFG_ERR_OOM, "pivoted Cholesky ERI decomposition: the ERI supermatrix does not fit");
   }
-  CK(diag.alloc(np));
-  CK(col.alloc(np));
-  CK(bad.alloc(1));
+  CK(diag.alloc(2 * (size_t)np));
   rc = eri_packed_locked(ctx, 1e-15, V.p, vlen);
   if (rc != HFG_OK) return rc;
   const unsigned g = (unsigned)std::min<long long>((np + 255) / 256, 4096);
   chol_diag_kernel<<<g, 256, 0, st>>>(V.p, np, diag.p);
   CK(cudaGetLastError());
-  CK(cudaMemsetAsync(bad.p, 0, 4, st));
   std::vector<double> d(np);
   CK(cudaMemcpyAsync(d.data(), diag.p, np * 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -116,38 +268,38 @@ extern "C" int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, h
   std::vector<long long> piv;
   long long rank = 0;
   double maxres = 0.0;
-  for (;;) {
-    double largest = -INFINITY;
-    for (double x : d) largest = std::max(largest, x);
-    long long pivot = 0;
-    while (!(d[pivot] >= largest - 1e-12 * std::fabs(largest))) ++pivot;
-    const double maximum = d[pivot];
-    if (maximum <= threshold || rank == np) {
-      maxres = std::max(maximum, 0.0);
-      break;
-    }
-    if (8.0 * (double)np * (double)(rank + 2) > (double)budget || rank >= cap)
-      return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: factor storage exceeds the memory budget");
-    const double root = std::sqrt(maximum);
-    double* row = df->B64.p + (size_t)rank * np;
-    chol_column_kernel<<<g, 256, 0, st>>>(V.p, np, pivot, row);
-    CK(cudaGetLastError());
-    if (rank > 0) {
-      // row -= sum_K L_K L_K[pivot]: L column-major (np x rank, ld np), x = L[:, pivot] (stride np)
-      const double m1 = -1.0, one = 1.0;
-      if (cublasDgemv(df->blas, CUBLAS_OP_N, (int)np, (int)rank, &m1, df->B64.p, (int)np, df->B64.p + pivot, (int)np,
-                      &one, row, 1) != CUBLAS_STATUS_SUCCESS)
-        return set_error(ctx, HFG_ERR_CUDA, "Cholesky projection GEMV");
-    }
-    chol_update_kernel<<<g, 256, 0, st>>>(row, np, pivot, root, scale, diag.p, bad.p);
-    CK(cudaGetLastError());
-    int hbad = 0;
-    CK(cudaMemcpyAsync(d.data(), diag.p, np * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&hbad, bad.p, 4, cudaMemcpyDeviceToHost, st));
+  {
+    DevBuf<double> bmax;
+    DevBuf<CholState> state;
+    DevBuf<long long> dpiv;
+    int sms = 148, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chol_kernel, kCholThreads, 0));
+    // one block per SM, at least one tile of columns each
+    const int blocks = (int)std::max<long long>(1, std::min<long long>(per_sm > 0 ? sms : 1, (np + kCholCols - 1) / kCholCols));
+    CK(bmax.alloc(2 * (size_t)blocks));
+    CK(state.alloc(1));
+    CK(dpiv.alloc((size_t)cap));
+    CK(cudaMemsetAsync(state.p, 0, sizeof(CholState), st));
+    long long per = (np + blocks - 1) / blocks;
+    per = (per + kCholCols - 1) / kCholCols * kCholCols;
+    CholArgs a{V.p, df->B64.p, diag.p, bmax.p, state.p, dpiv.p, np, cap, per, threshold, scale, (double)budget};
+    void* args[] = {&a};
+    CK(cudaLaunchCooperativeKernel((const void*)chol_kernel, dim3((unsigned)blocks), dim3(kCholThreads), args, 0, st));
+    CholState h{};
+    CK(cudaMemcpyAsync(&h, state.p, sizeof(h), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (hbad) return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: nonpositive residual Coulomb diagonal");
-    piv.push_back(pivot);
-    ++rank;
+    if (h.status == 3)
+      return set_error(ctx, HFG_ERR_TIMEOUT, "pivoted Cholesky ERI decomposition: a bounded wait ran out");
+    if (h.status == 2)
+      return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: factor storage exceeds the memory budget");
+    if (h.bad)
+      return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: nonpositive residual Coulomb diagonal");
+    rank = h.rank;
+    maxres = h.residual;
+    piv.resize((size_t)rank);
+    if (rank > 0) CK(cudaMemcpyAsync(piv.data(), dpiv.p, (size_t)rank * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
   }
   if (rank == 0)
     return set_error(ctx, HFG_ERR_INTEGRAL,

@@ -1577,17 +1577,29 @@ int eri_packed_locked(hfg_ctx* ctx, double thr, double* d_out, size_t len) {
   int rc = build_plan(ctx, thr, 0.0, 0.0, HFG_FP64, 0, kPlanWhole, plan);
   if (rc != HFG_OK) return rc;
   HFG_CUDA(ctx, cudaMemsetAsync(d_out, 0, len * sizeof(double), ctx->stream));
-  for (const Launch& L : plan->launches) {
-    if (L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax) {
-      HFG_CUDA(ctx, launch_eri_packed_md(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0],
-                                         L.prefix[1], ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p,
-                                         ctx->d_pbound.p, ctx->d_boys64.p, ctx->d_expt64.p, d_out, ctx->stream));
-      continue;
-    }
-    HFG_CUDA(ctx, launch_eri_packed(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0], L.prefix[1],
-                                    ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p, ctx->d_boys64.p, ctx->d_expt64.p, d_out,
-                                    ctx->stream));
+  // the classes write different slots: they run concurrently over the context
+  // stream and its side streams
+  HFG_CUDA(ctx, ctx->ensure_side_streams());
+  HFG_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ctx->stream));
+  for (int k = 0; k < kJKSideStreams; ++k) HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
+  cudaError_t le = cudaSuccess;
+  for (size_t l = 0; l < plan->launches.size() && le == cudaSuccess; ++l) {
+    const Launch& L = plan->launches[l];
+    const size_t si = l % (1 + kJKSideStreams);
+    cudaStream_t ls = si == 0 ? ctx->stream : ctx->side[si - 1];
+    const bool md = L.coop || L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
+    le = md ? launch_eri_packed_md(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0], L.prefix[1],
+                                   ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p, ctx->d_pbound.p,
+                                   ctx->d_boys64.p, ctx->d_expt64.p, d_out, ls)
+            : launch_eri_packed(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0], L.prefix[1],
+                                ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p, ctx->d_boys64.p,
+                                ctx->d_expt64.p, d_out, ls);
   }
+  for (int k = 0; k < kJKSideStreams; ++k) {
+    HFG_CUDA(ctx, cudaEventRecord(ctx->ev_join[k], ctx->side[k]));
+    HFG_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_join[k], 0));
+  }
+  HFG_CUDA(ctx, le);
   return HFG_OK;
 }
 }  // namespace hfg
