@@ -111,20 +111,22 @@ int ensure_tiles(hfg_df* df, int kind) {
   if (rc != HFG_OK) return rc;
   TileStructure& t = df->tiles[kind];
   t.build(colmn, df->n, kind);
-  auto up = [&](DevBuf<int>& d, const std::vector<int>& h) -> int {
+  auto up = [&](auto& d, const auto& h) -> int {
     int r = cuda_check(ctx, d.alloc(std::max<size_t>(1, h.size())), "alloc tile structure");
     if (r == HFG_OK && !h.empty())
-      r = cuda_check(ctx, cudaMemcpyAsync(d.p, h.data(), h.size() * 4, cudaMemcpyHostToDevice, ctx->stream),
+      r = cuda_check(ctx, cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, ctx->stream),
                      "copy tile structure");
     return r;
   };
   if ((rc = up(df->tile_off[kind], t.tile_off)) != HFG_OK) return rc;
   if ((rc = up(df->tile_kt[kind], t.tile_kt)) != HFG_OK) return rc;
-  if ((rc = up(df->tile_map[kind], t.tile_map)) != HFG_OK) return rc;
+  if ((rc = up(df->list_off[kind], t.list_off)) != HFG_OK) return rc;
+  if ((rc = up(df->list_col[kind], t.list_col)) != HFG_OK) return rc;
+  if ((rc = up(df->list_pos[kind], t.list_pos)) != HFG_OK) return rc;
   rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "tile structure");
   if (rc != HFG_OK) return rc;
-  t.tile_map.clear();
-  t.tile_map.shrink_to_fit();
+  t.list_col = {};
+  t.list_pos = {};
   df->tiles_ready[kind] = true;
   return HFG_OK;
 }
@@ -526,7 +528,9 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
     ua.tiles = &df->tiles[kind];
     ua.tile_off_dev = df->tile_off[kind].p;
     ua.tile_kt_dev = df->tile_kt[kind].p;
-    ua.tile_map_dev = df->tile_map[kind].p;
+    ua.list_off_dev = df->list_off[kind].p;
+    ua.list_col_dev = df->list_col[kind].p;
+    ua.list_pos_dev = df->list_pos[kind].p;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     ua.chunk_bytes = std::max<size_t>((size_t)64 << 20, std::min<size_t>((size_t)4 << 30, free_b / 4));

@@ -31,7 +31,8 @@ struct hfg_df {
   // type (built on first use) and its scratch
   hfg::TileStructure tiles[2];
   bool tiles_ready[2] = {false, false};
-  hfg::DevBuf<int> tile_off[2], tile_kt[2], tile_map[2];
+  hfg::DevBuf<int> tile_off[2], tile_kt[2], list_off[2], list_col[2];
+  hfg::DevBuf<unsigned short> list_pos[2];
   hfg::UmmaWorkspace uws;
   // device time of the last exchange (K) and its executed tensor-core flops
   cudaEvent_t kev[2] = {nullptr, nullptr};

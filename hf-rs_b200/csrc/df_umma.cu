@@ -20,8 +20,8 @@
 //                an n x n FP32 accumulator.
 //
 // Both GEMMs are one warp-specialised kernel: warp 0 issues TMA tile loads
-// (cp.async.bulk.tensor, 128-byte swizzle) into a 4-stage shared-memory
-// ring, warp 1 allocates TMEM and issues tcgen05.mma (one elected thread;
+// (cp.async.bulk.tensor, 128-byte swizzle) into a shared-memory ring of 4 to
+// 8 stages (as many as the launch's tile width leaves room for), warp 1 allocates TMEM and issues tcgen05.mma (one elected thread;
 // M = 128, N = up to 256, K = 16 (BF16) or 8 (TF32) per instruction) and
 // releases ring slots with tcgen05.commit, warps 2-5 read the accumulator
 // back with tcgen05.ld and store it.  All tensor maps cover this GPU's own
@@ -45,7 +45,7 @@
 namespace hfg {
 namespace umma {
 
-constexpr int kStages = 4;
+constexpr int kMaxStages = 8;
 constexpr int kBM = 128;
 constexpr int kBN = 256;
 constexpr int kRowBytes = 128;  // one swizzle span: BK elements of the operand type
@@ -53,8 +53,15 @@ constexpr int kThreads = 192;   // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 constexpr int kTmemCols = 256;
 
 constexpr int kStageA = kBM * kRowBytes;  // 16 KB
-constexpr int kStageB = kBN * kRowBytes;  // 32 KB
-constexpr size_t kSmemBytes = (size_t)kStages * (kStageA + kStageB) + 1024 /*align*/ + 256 /*barriers*/;
+constexpr size_t kSmemSlack = 1024 /*align*/ + 256 /*barriers*/;
+constexpr size_t kSmemMax = 227 * 1024;
+// A stage holds one A tile and one B tile of `box` rows: T = B_Q C with few
+// occupied orbitals loads only the columns it multiplies (a box of 256 rows
+// for 128 of them spent half the loads on zeros and a third of the ring), and
+// the smaller stages make the ring deeper, which its HBM latency needs.
+inline int stage_count(int box) {
+  return (int)std::min<size_t>(kMaxStages, (kSmemMax - kSmemSlack) / (kStageA + (size_t)box * kRowBytes));
+}
 
 // ------------------------------------------------------------ PTX helpers --
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -86,11 +93,16 @@ __device__ __forceinline__ uint64_t global_ns() {
 // in a working kernel lasts at most one output tile's main loop (well under
 // a millisecond).
 constexpr uint64_t kWaitNs = 2000000000ull;
+// The clock is first read after 256 polls: a read costs more than most waits.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;
   for (uint32_t i = 0;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && (*abort || global_ns() - t0 > kWaitNs)) return false;
+    if ((i & 255u) == 255u) {
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      if (*abort || now - t0 > kWaitNs) return false;
+    }
   }
 }
 // Drain-only wait (no abort check): lets this block's own in-flight copies
@@ -206,6 +218,8 @@ struct GemmArgs {
   int m_rows;  // valid rows of the output (n)
   int n_cols;  // valid columns of the output (mode 0: nocc_pad; mode 1: n)
   int bn;      // output tile width (<= 256, multiple of 16)
+  int box;     // rows of the B tile's TMA box (>= bn, multiple of 16)
+  int stages;  // ring stages
   long long units;  // work units of the launch
   // mode 0: unit = (nt, mt, Q), nt fastest
   const int* tile_off;  // per row block: its non-zero tiles [tile_off[mt], tile_off[mt + 1])
@@ -264,11 +278,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int kEl = KIND == kBF16 ? 2 : 4;  // operand bytes; 32 bytes of K per instruction
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int stages = a.stages, stageB = a.box * kRowBytes;
   unsigned char* sA = base;
-  unsigned char* sB = base + kStages * kStageA;
-  uint64_t* full = (uint64_t*)(sB + kStages * kStageB);
-  uint64_t* empty = full + kStages;
-  uint64_t* tfull = empty + kStages;  // accumulator buffer b holds a finished unit
+  unsigned char* sB = base + stages * kStageA;
+  uint64_t* full = (uint64_t*)(sB + stages * stageB);
+  uint64_t* empty = full + kMaxStages;
+  uint64_t* tfull = empty + kMaxStages;  // accumulator buffer b holds a finished unit
   uint64_t* tempty = tfull + 2;       // accumulator buffer b has been read out
   uint64_t* done = tempty + 2;
   uint32_t* tmem_slot = (uint32_t*)(done + 1);
@@ -276,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -299,16 +314,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------- producer
-    int last_round[kStages];
-#pragma unroll
-    for (int s = 0; s < kStages; ++s) last_round[s] = -1;
-    const uint32_t bytes = (uint32_t)(kStageA + kStageB);
-    long long it = 0;
+    const uint32_t bytes = (uint32_t)(kStageA + stageB);
+    int s = 0, first = 1;  // slot, and whether this is the ring's first round
+    uint32_t round = 0;
     for (long long u = blockIdx.x; u < a.units && !*abort_flag; u += gridDim.x) {
       const Unit w = unit_of<MODE>(a, u);
-      for (int k = 0; k < w.nk; ++k, ++it) {
-        const int s = (int)(it % kStages);
-        const uint32_t round = (uint32_t)(it / kStages);
+      for (int k = 0; k < w.nk; ++k) {
         if (!mbar_wait(&empty[s], (round & 1u) ^ 1u, abort_flag)) {
           if (!*abort_flag) atomicExch(a.err, 1);
           *abort_flag = 1;
@@ -332,17 +343,24 @@ __global__ void __launch_bounds__(kThreads, 1)
           az = bz = q;
         }
         tma_load_3d(sA + s * kStageA, &tmA, &full[s], ax, ay, az);
-        tma_load_3d(sB + s * kStageB, &tmB, &full[s], bx, by, bz);
-        last_round[s] = (int)round;
+        tma_load_3d(sB + s * stageB, &tmB, &full[s], bx, by, bz);
+        if (++s == stages) {
+          s = 0;
+          first = 0;
+          ++round;
+        }
       }
     }
-    // let every copy this thread issued land before the block may exit
-    for (int s = 0; s < kStages; ++s)
-      if (last_round[s] >= 0 && !mbar_wait_drain(&full[s], (uint32_t)(last_round[s] & 1))) atomicExch(a.err, 2);
+    // let every copy this thread issued land before the block may exit:
+    // slots below s were last filled in this round, the others in the last
+    for (int t = 0; t < stages; ++t) {
+      if (t >= s && first) continue;
+      if (!mbar_wait_drain(&full[t], (t < s ? round : round - 1) & 1u)) atomicExch(a.err, 2);
+    }
   } else if (warp == 1 && lane == 0) {
     // ------------------------------------------------------- MMA issuer
-    long long it = 0;
-    int lt = 0;
+    int s = 0, lt = 0;
+    uint32_t round = 0;
     for (long long u = blockIdx.x; u < a.units && !*abort_flag; u += gridDim.x, ++lt) {
       const Unit w = unit_of<MODE>(a, u);
       const int b = lt & 1;
@@ -356,9 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t d = tmem + (uint32_t)(b * kTmemCols);
       const uint32_t idesc = make_idesc(kFmt, kBM, (uint32_t)unit_cols(a, w));
       bool ok = true;
-      for (int k = 0; k < w.nk; ++k, ++it) {
-        const int s = (int)(it % kStages);
-        const uint32_t round = (uint32_t)(it / kStages);
+      for (int k = 0; k < w.nk; ++k) {
         if (!mbar_wait(&full[s], round & 1u, abort_flag)) {
           if (!*abort_flag) atomicExch(a.err, 4);
           *abort_flag = 1;
@@ -366,11 +382,15 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         tc_fence_after();
-        const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sB + s * kStageB);
+        const uint32_t a0 = smem_u32(sA + s * kStageA), b0 = smem_u32(sB + s * stageB);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)  // 4 x 32 bytes of K per 128-byte row
           umma<KIND>(d, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), idesc, (k > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&empty[s]);  // the slot is free once these MMAs have read it
+        if (++s == stages) {
+          s = 0;
+          ++round;
+        }
       }
       if (!ok) break;
       umma_commit(&tfull[b]);  // with no MMAs (nk = 0) it arrives at once
@@ -449,30 +469,59 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ----------------------------------------------------------------- unpack --
-// Tile-compact unpack: block = one non-zero 128 x TK tile of the row-block
-// structure; each thread keeps its elements' packed-column indices and walks
-// the Q of the chunk.  dst[Q][tile][r][c] (row stride TK).
-template <typename TS, typename TD, int TK>
+// Tile-compact unpack, dst[Q][tile][r][c] (row stride TK): block = half of
+// one non-zero 128 x TK tile (64 rows) and every gridDim.y-th Q of the chunk.
+// The half's elements are listed in the order of their packed columns, so a
+// warp reads runs of consecutive columns (whole shell-pair blocks; an
+// element-ordered gather touches a cache line per row of each block), places
+// them in a shared-memory image, and the image goes out in 16-byte stores.
+// The next Q's values are in flight meanwhile.  The image's 16-byte units are
+// swizzled by row (unit ^ row % 8, as the list's positions are), or the rows
+// of a block, 128 bytes apart, would share their banks.  Elements outside the
+// list stay zero from the start.
+template <typename TS, typename TD>
 __global__ void __launch_bounds__(256) unpack_tiles_kernel(const TS* __restrict__ B, long long ncol,
-                                                           const int* __restrict__ tile_map, int ntiles, int q0,
-                                                           int qn, TD* __restrict__ dst) {
-  constexpr int kPer = kBM * TK / 256;
-  const int t = blockIdx.x;
-  if (t >= ntiles) return;
-  const int* m = tile_map + (size_t)t * kBM * TK;
-  int idx[kPer];
+                                                           const int* __restrict__ list_off,
+                                                           const int* __restrict__ list_col,
+                                                           const unsigned short* __restrict__ list_pos, int halves,
+                                                           int q0, int qn, TD* __restrict__ dst) {
+  constexpr int kHalf = kBM / 2 * kRowBytes / (int)sizeof(TD), kPer = kHalf / 256, kUnits = kHalf * (int)sizeof(TD) / 16;
+  __shared__ __align__(16) TD img[2][kHalf];
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int l0 = list_off[t], ln = list_off[t + 1] - l0;
+  int col[kPer];
+  unsigned short pos[kPer];
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) idx[k] = __ldg(m + threadIdx.x + k * 256);
-  for (int q = blockIdx.y; q < qn; q += gridDim.y) {
+  for (int k = 0; k < kPer; ++k) {
+    const int x = tid + k * 256;
+    col[k] = x < ln ? __ldg(list_col + l0 + x) : -1;
+    pos[k] = x < ln ? __ldg(list_pos + l0 + x) : (unsigned short)0;
+  }
+  for (int x = tid; x < 2 * kUnits; x += 256) ((uint4*)img)[x] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  TS cur[kPer], nxt[kPer];
+  auto fetch = [&](int q, TS* v) {
     const TS* row = B + (size_t)(q0 + q) * ncol;
-    TD* o = dst + ((size_t)q * ntiles + t) * kBM * TK;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const int e = idx[k];
-      float v = 0.f;
-      if (e >= 0) v = (float)row[e];
-      o[threadIdx.x + k * 256] = to_operand<TD>(v);
-    }
+    for (int k = 0; k < kPer; ++k)
+      if (col[k] >= 0) v[k] = row[col[k]];
+  };
+  int q = blockIdx.y, b = 0;
+  if (q < qn) fetch(q, cur);
+  for (; q < qn; q += gridDim.y, b ^= 1) {
+    if (q + (int)gridDim.y < qn) fetch(q + gridDim.y, nxt);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (col[k] >= 0) img[b][pos[k]] = to_operand<TD>((float)cur[k]);
+    __syncthreads();
+    // (the image written two rounds ago is rewritten only after the next
+    // barrier, which every thread reaches after its stores from it)
+    uint4* o = (uint4*)(dst + ((size_t)q * halves + t) * kHalf);
+    const uint4* m = (const uint4*)img[b];
+#pragma unroll
+    for (int x = tid; x < kUnits; x += 256) o[x] = m[(x & ~7) | ((x ^ (x >> 3)) & 7)];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) cur[k] = nxt[k];
   }
 }
 
@@ -535,8 +584,9 @@ static cudaError_t launch_gemm(const CUtensorMap& A, const CUtensorMap& B, const
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64)
-    std::call_once(once[dev], [&] { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes); });
-  k<<<grid, kThreads, kSmemBytes, st>>>(A, B, a);
+    std::call_once(once[dev], [&] { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax); });
+  const size_t smem = (size_t)a.stages * (kStageA + (size_t)a.box * kRowBytes) + kSmemSlack;
+  k<<<grid, kThreads, smem, st>>>(A, B, a);
   return cudaGetLastError();
 }
 
@@ -546,41 +596,48 @@ using namespace umma;
 
 int TileStructure::build(const std::vector<int2>& colmn, int n, int kind) {
   this->n = n;
-  tk = kind == kBF16 ? 64 : 32;
+  const unsigned ks = kind == kBF16 ? 6 : 5;  // log2 of a tile's columns
+  tk = 1 << ks;
   const int nmt = (n + kBM - 1) / kBM, nkt = (n + tk - 1) / tk;
-  // packed column of every (row, col) of B_Q, -1 where no significant pair
-  std::vector<int> full((size_t)n * n, -1);
-  for (size_t c = 0; c < colmn.size(); ++c) {
-    const int i = colmn[c].x, j = colmn[c].y;
-    full[(size_t)i * n + j] = (int)c;
-    full[(size_t)j * n + i] = (int)c;
-  }
-  std::vector<char> nz((size_t)nmt * nkt, 0);
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j)
-      if (full[(size_t)i * n + j] >= 0) nz[(size_t)(i / kBM) * nkt + j / tk] = 1;
+  // f(row block, row in block, column) of every element of column c of B_Q
+  auto each = [&](size_t c, auto&& f) {
+    const unsigned i = colmn[c].x, j = colmn[c].y;
+    f(i / kBM, i % kBM, j);
+    if (i != j) f(j / kBM, j % kBM, i);
+  };
+  std::vector<int> tile((size_t)nmt * nkt, 0);
+  for (size_t c = 0; c < colmn.size(); ++c)
+    each(c, [&](unsigned mt, unsigned, unsigned j) { tile[(size_t)mt * nkt + (j >> ks)] = 1; });
   tile_off.assign(nmt + 1, 0);
   tile_kt.clear();
   for (int mt = 0; mt < nmt; ++mt) {
     for (int kt = 0; kt < nkt; ++kt)
-      if (nz[(size_t)mt * nkt + kt]) tile_kt.push_back(kt);
+      if (tile[(size_t)mt * nkt + kt]) {
+        tile[(size_t)mt * nkt + kt] = (int)tile_kt.size();
+        tile_kt.push_back(kt);
+      }
     tile_off[mt + 1] = (int)tile_kt.size();
   }
   ntiles = (int)tile_kt.size();
-  tile_map.assign((size_t)ntiles * kBM * tk, -1);
-  for (int mt = 0; mt < nmt; ++mt)
-    for (int t = tile_off[mt]; t < tile_off[mt + 1]; ++t) {
-      const int kt = tile_kt[t];
-      for (int r = 0; r < kBM; ++r) {
-        const int i = mt * kBM + r;
-        if (i >= n) break;
-        for (int c = 0; c < tk; ++c) {
-          const int j = kt * tk + c;
-          if (j >= n) break;
-          tile_map[((size_t)t * kBM + r) * tk + c] = full[(size_t)i * n + j];
-        }
-      }
-    }
+  // per half tile: its elements (packed column, swizzled position) in the
+  // columns' order, counted and then placed (the first exchange of a factor
+  // waits for these lists: sorting them took 8 ms at n = 480)
+  // (a 128-byte row of a tile holds eight units of 16 bytes)
+  auto half = [&](unsigned mt, unsigned r, unsigned j) { return 2 * tile[(size_t)mt * nkt + (j >> ks)] + r / (kBM / 2); };
+  list_off.assign(2 * ntiles + 1, 0);
+  for (size_t c = 0; c < colmn.size(); ++c)
+    each(c, [&](unsigned mt, unsigned r, unsigned j) { ++list_off[half(mt, r, j) + 1]; });
+  for (int h = 0; h < 2 * ntiles; ++h) list_off[h + 1] += list_off[h];
+  list_col.resize(list_off[2 * ntiles]);
+  list_pos.resize(list_off[2 * ntiles]);
+  std::vector<int> at(list_off.begin(), list_off.end() - 1);
+  for (size_t c = 0; c < colmn.size(); ++c)
+    each(c, [&](unsigned mt, unsigned r, unsigned j) {
+      const int x = at[half(mt, r, j)]++;
+      const unsigned rh = r % (kBM / 2), cc = j & (tk - 1), us = ks - 3;
+      list_col[x] = (int)c;
+      list_pos[x] = (unsigned short)((rh << ks) + (((cc >> us) ^ (rh & 7)) << us) + (cc & ((1u << us) - 1)));
+    });
   total_tiles = nmt * nkt;
   return 0;
 }
@@ -625,8 +682,12 @@ cudaError_t df_k_tensor_cores(const UmmaDfArgs& p, UmmaWorkspace& ws, int* statu
   if ((e = cudaMemcpyAsync(ws.lower.p, lower.data(), lower.size() * sizeof(int2), cudaMemcpyHostToDevice, st)) !=
       cudaSuccess)
     return e;
+  // GEMM 1: equal column tiles of at most 256 (a narrow remainder tile would
+  // run the tensor cores below their rate), loaded in boxes of their width
+  const int n_ntiles = (nocc_pad + kBN - 1) / kBN;
+  const int bn1 = ((nocc_pad + n_ntiles - 1) / n_ntiles + 15) / 16 * 16;
   CUtensorMap mCt, mA1, mT_A, mT_B;
-  if (!make_map(&mCt, kind, ws.Ct.p, ldk, nocc_pad, 1, (long long)ldk * el, (long long)nocc_pad * ldk * el, kBN))
+  if (!make_map(&mCt, kind, ws.Ct.p, ldk, nocc_pad, 1, (long long)ldk * el, (long long)nocc_pad * ldk * el, bn1))
     return cudaErrorInvalidValue;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
@@ -652,20 +713,20 @@ cudaError_t df_k_tensor_cores(const UmmaDfArgs& p, UmmaWorkspace& ws, int* statu
     if (profile) cudaEventRecord(pev[0], st);
     // 1. unpack the chunk's non-zero tiles
     {
-      dim3 g((unsigned)ts.ntiles, (unsigned)std::min(qn, 64));
+      dim3 g((unsigned)(2 * ts.ntiles), (unsigned)std::min(qn, 64));
       if (ts.ntiles > 0) {
-        if (kind == kBF16) {
-          if (p.storage == 1)
-            unpack_tiles_kernel<float, __nv_bfloat16, 64><<<g, 256, 0, st>>>(
-                (const float*)p.B, p.ncol, p.tile_map_dev, ts.ntiles, p.rank_offset + q0, qn, (__nv_bfloat16*)ws.dense.p);
-          else
-            unpack_tiles_kernel<__nv_bfloat16, __nv_bfloat16, 64><<<g, 256, 0, st>>>(
-                (const __nv_bfloat16*)p.B, p.ncol, p.tile_map_dev, ts.ntiles, p.rank_offset + q0, qn,
-                (__nv_bfloat16*)ws.dense.p);
-        } else {
-          unpack_tiles_kernel<float, float, 32><<<g, 256, 0, st>>>((const float*)p.B, p.ncol, p.tile_map_dev,
-                                                                   ts.ntiles, p.rank_offset + q0, qn, (float*)ws.dense.p);
-        }
+        const int r0 = p.rank_offset + q0;
+        if (kind == kBF16 && p.storage == 1)
+          unpack_tiles_kernel<float, __nv_bfloat16><<<g, 256, 0, st>>>((const float*)p.B, p.ncol, p.list_off_dev,
+                                                                       p.list_col_dev, p.list_pos_dev, 2 * ts.ntiles, r0, qn,
+                                                                       (__nv_bfloat16*)ws.dense.p);
+        else if (kind == kBF16)
+          unpack_tiles_kernel<__nv_bfloat16, __nv_bfloat16><<<g, 256, 0, st>>>(
+              (const __nv_bfloat16*)p.B, p.ncol, p.list_off_dev, p.list_col_dev, p.list_pos_dev, 2 * ts.ntiles, r0, qn,
+              (__nv_bfloat16*)ws.dense.p);
+        else
+          unpack_tiles_kernel<float, float><<<g, 256, 0, st>>>((const float*)p.B, p.ncol, p.list_off_dev, p.list_col_dev,
+                                                               p.list_pos_dev, 2 * ts.ntiles, r0, qn, (float*)ws.dense.p);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
       }
     }
@@ -684,10 +745,9 @@ cudaError_t df_k_tensor_cores(const UmmaDfArgs& p, UmmaWorkspace& ws, int* statu
     g1.ldo = nocc_pad;
     g1.batch_stride = (long long)n * nocc_pad;
     g1.err = (int*)ws.err.p;
-    // equal column tiles of at most 256 (a narrow remainder tile would run
-    // the tensor cores below their rate)
-    g1.n_ntiles = (nocc_pad + kBN - 1) / kBN;
-    g1.bn = ((nocc_pad + g1.n_ntiles - 1) / g1.n_ntiles + 15) / 16 * 16;
+    g1.n_ntiles = n_ntiles;
+    g1.bn = g1.box = bn1;
+    g1.stages = stage_count(bn1);
     g1.n_mtiles = nmt;
     g1.units = (long long)g1.n_ntiles * nmt * qn;
     dim3 grid1((unsigned)std::min<long long>(g1.units, sms));
@@ -707,7 +767,8 @@ cudaError_t df_k_tensor_cores(const UmmaDfArgs& p, UmmaWorkspace& ws, int* statu
     g2.mode = 1;
     g2.m_rows = n;
     g2.n_cols = n;
-    g2.bn = kBN;
+    g2.bn = g2.box = kBN;
+    g2.stages = stage_count(kBN);
     g2.out_tiles = (const int2*)ws.lower.p;
     g2.n_lower = (int)lower.size();
     g2.q_count = qn;

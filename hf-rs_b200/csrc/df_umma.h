@@ -14,11 +14,13 @@ constexpr int kBF16 = 0, kTF32 = 1;  // operand type of both exchange GEMMs
 // Non-zero 128 x TK tiles of B_Q (the same for every Q): the AO pairs stored
 // in the factor decide which tiles of the symmetric n x n unpack hold
 // anything.  tile_off[mt] .. tile_off[mt + 1] are the tiles of row block mt
-// (column blocks tile_kt[]); tile_map holds, per tile, the packed factor
-// column of each of its 128 x TK elements (-1: zero).
+// (column blocks tile_kt[]); elements [list_off[h], list_off[h + 1]) of the
+// lists are the packed factor columns of half tile h (64 rows of tile h / 2),
+// ascending, and their positions in its swizzled image (unpack_tiles_kernel).
 struct TileStructure {
   int n = 0, tk = 0, ntiles = 0, total_tiles = 0;
-  std::vector<int> tile_off, tile_kt, tile_map;
+  std::vector<int> tile_off, tile_kt, list_off, list_col;
+  std::vector<unsigned short> list_pos;
   int build(const std::vector<int2>& colmn, int n, int kind);
 };
 
@@ -42,7 +44,9 @@ struct UmmaDfArgs {
   const TileStructure* tiles = nullptr;
   const int* tile_off_dev = nullptr;
   const int* tile_kt_dev = nullptr;
-  const int* tile_map_dev = nullptr;
+  const int* list_off_dev = nullptr;
+  const int* list_col_dev = nullptr;
+  const unsigned short* list_pos_dev = nullptr;
   size_t chunk_bytes = (size_t)4 << 30;  // scratch for one chunk of Q
   int max_chunk = 0;                      // > 0: at most this many Q per chunk
 };
