@@ -447,6 +447,14 @@ int hfg_df_three_center(hfg_ctx* ctx, const hfg_basis* aux, double* out, size_t 
 
 }  // extern "C"
 
+int hfg_df::ensure_map() {
+  if (map.p) return HFG_OK;
+  int rc = cuda_check(ctx, map.alloc((size_t)n * n), "alloc pair map");
+  if (rc == HFG_OK) rc = cuda_check(ctx, launch_df_map(colmn.p, ncol, n, map.p, ctx->stream), "pair map");
+  if (rc != HFG_OK) map.release();
+  return rc;
+}
+
 namespace hfg {
 
 bool df_is_shard(const hfg_df* df) { return df->shard(); }
@@ -560,17 +568,18 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
   const size_t budget = std::max<size_t>((size_t)64 << 20, std::min<size_t>((size_t)4 << 30, free_b / 4));
   int qc = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(rank, 1), budget / ((size_t)nn * esz)));
   CK(df->dense.alloc((size_t)qc * nn * esz));
+  rc = df->ensure_map();
+  if (rc != HFG_OK) return rc;
   CK(cudaMemsetAsync(dK, 0, nn * 8, st));
   if (mma == HFG_DF_FP64) {
     CK(df->T64.alloc((size_t)qc * n * nocc));
     for (int q0 = q_lo; q0 < q_hi; q0 += qc) {
       const int qn = std::min(qc, q_hi - q0);
-      CK(cudaMemsetAsync(df->dense.p, 0, (size_t)qn * nn * 8, st));
       // FP64 arithmetic on the stored factor, converted while unpacking
       const int um = df->storage == HFG_DF_FP64 ? 0 : (df->storage == HFG_DF_FP32 ? 3 : 4);
       const void* Bs = df->storage == HFG_DF_FP64 ? (const void*)df->B64.p
                        : df->storage == HFG_DF_FP32 ? (const void*)df->B32.p : (const void*)df->B16.p;
-      CK(launch_df_unpack(um, Bs, ncol, df->colmn.p, ncol, q0, qn, n, df->dense.p, st));
+      CK(launch_df_unpack(um, Bs, ncol, df->map.p, q0, qn, n, df->dense.p, st));
       const double* Bd = (const double*)df->dense.p;
       // T^T (nocc x n*qn) = C^T (nocc x n) * Bd2^T (n x n*qn)
       cublasDgemm(df->blas, CUBLAS_OP_T, CUBLAS_OP_N, nocc, n * qn, n, &one, dC, n, Bd, n, &zero, df->T64.p, nocc);
@@ -599,8 +608,7 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
     const int umode = df->storage == HFG_DF_BF16 ? 2 : (bf ? 5 : 1);
     for (int q0 = q_lo; q0 < q_hi; q0 += qc) {
       const int qn = std::min(qc, q_hi - q0);
-      CK(cudaMemsetAsync(df->dense.p, 0, (size_t)qn * nn * esz, st));
-      CK(launch_df_unpack(umode, Bsrc, ncol, df->colmn.p, ncol, q0, qn, n, df->dense.p, st));
+      CK(launch_df_unpack(umode, Bsrc, ncol, df->map.p, q0, qn, n, df->dense.p, st));
       rc = gemm_ex(ctx, df->blas, CUBLAS_OP_T, CUBLAS_OP_N, nocc, n * qn, n, Cin, it, n, df->dense.p, it, n, 0.0f,
                    df->Tf.p, nocc, ct);
       if (rc != HFG_OK) return rc;

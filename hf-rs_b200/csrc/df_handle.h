@@ -21,6 +21,9 @@ struct hfg_df {
   hfg::DevBuf<float> B32;
   hfg::DevBuf<__nv_bfloat16> B16;
   hfg::DevBuf<int2> colmn;
+  hfg::DevBuf<int> map;  // packed column of every AO pair (n x n, -1: none), made on first use
+  // (in hfg_df's context, lock held)
+  int ensure_map();
   hfg::DevBuf<double> metric;  // kept for inspection (naux x naux)
   cublasHandle_t blas = nullptr;
   hfg::DevBuf<double> P, pvec, gam, jcol, Cd, J, K, T64;

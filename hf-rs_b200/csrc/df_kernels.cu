@@ -135,62 +135,65 @@ cudaError_t launch_df3c(int la, int lb, int lc, const Df3cArgs& args, cudaStream
   return cudaErrorInvalidValue;
 }
 
+// Packed column of every (m, k) of B_Q into map (n x n, preset to -1).
+__global__ void df_map_kernel(const int2* __restrict__ colmn, long long ncol, int n, int* __restrict__ map) {
+  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncol; c += (long long)gridDim.x * blockDim.x) {
+    const int2 mn = colmn[c];
+    map[(size_t)mn.x * n + mn.y] = (int)c;
+    map[(size_t)mn.y * n + mn.x] = (int)c;
+  }
+}
+
+cudaError_t launch_df_map(const int2* colmn, long long ncol, int n, int* map, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(map, 0xff, (size_t)n * n * 4, st);
+  if (e != cudaSuccess || ncol <= 0) return e;
+  df_map_kernel<<<(unsigned)std::min<long long>((ncol + 255) / 256, 148 * 8), 256, 0, st>>>(colmn, ncol, n, map);
+  return cudaGetLastError();
+}
+
 // Unpack rows [q0, q0+qc) of B (rank x ncol, packed unique AO pairs) into
 // the dense layout out[(m * qc + q) * n + k] = B_q[m][k] (both triangles),
-// converted to the GEMM input type.
+// converted to the GEMM input type.  Every output element is written once,
+// zeros included, in coalesced rows that gather from B_q through the map
+// (a B_q row is re-read from L2); a scatter from the packed columns writes
+// each pair to two far places in pieces of a sector and needs the chunk
+// cleared first.  The block's threads keep their map entries over its Q.
 template <typename TO, typename TI>
-__global__ void df_unpack_kernel(const TI* __restrict__ B, long long ldb, const int2* __restrict__ colmn,
-                                 long long ncol, int q0, int qc, int n, TO* __restrict__ out) {
-  const long long total = ncol * qc;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(t / ncol);
-    const long long c = t % ncol;
-    const int2 mn = colmn[c];
-    const TO v = (TO)(float)B[(long long)(q0 + q) * ldb + c];
-    out[((long long)mn.x * qc + q) * n + mn.y] = v;
-    out[((long long)mn.y * qc + q) * n + mn.x] = v;
+__global__ void __launch_bounds__(256) df_unpack_kernel(const TI* __restrict__ B, long long ldb,
+                                                        const int* __restrict__ map, int q0, int qc, int n,
+                                                        TO* __restrict__ out) {
+  constexpr int kRows = 4;  // rows m of one block: a shell's rows share the sectors of its pair blocks
+  const int k = blockIdx.x * 64 + (threadIdx.x & 63), m = blockIdx.y * kRows + (threadIdx.x >> 6);
+  if (k >= n || m >= n) return;
+  const int c = __ldg(map + (size_t)m * n + k);
+#pragma unroll 4
+  for (int q = blockIdx.z; q < qc; q += gridDim.z) {
+    TO v = (TO)0.0f;
+    if (c >= 0) {
+      const TI x = B[(size_t)(q0 + q) * ldb + c];
+      if constexpr (sizeof(TI) == 8) v = x;
+      else v = (TO)(float)x;
+    }
+    out[((size_t)m * qc + q) * n + k] = v;
   }
 }
 
-template <>
-__global__ void df_unpack_kernel<double, double>(const double* __restrict__ B, long long ldb,
-                                                 const int2* __restrict__ colmn, long long ncol, int q0, int qc,
-                                                 int n, double* __restrict__ out) {
-  const long long total = ncol * qc;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(t / ncol);
-    const long long c = t % ncol;
-    const int2 mn = colmn[c];
-    const double v = B[(long long)(q0 + q) * ldb + c];
-    out[((long long)mn.x * qc + q) * n + mn.y] = v;
-    out[((long long)mn.y * qc + q) * n + mn.x] = v;
-  }
-}
-
-cudaError_t launch_df_unpack(int mode, const void* B, long long ldb, const int2* colmn, long long ncol, int q0, int qc,
-                             int n, void* out, cudaStream_t st) {
-  const long long total = ncol * qc;
-  const unsigned grid = (unsigned)std::min<long long>((total + 255) / 256, 148 * 32);
-  if (total <= 0) return cudaSuccess;
-  if (mode == 0)
-    df_unpack_kernel<double, double><<<grid, 256, 0, st>>>((const double*)B, ldb, colmn, ncol, q0, qc, n,
-                                                           (double*)out);
-  else if (mode == 1)
-    df_unpack_kernel<float, float><<<grid, 256, 0, st>>>((const float*)B, ldb, colmn, ncol, q0, qc, n, (float*)out);
-  else if (mode == 2)
-    df_unpack_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)B, ldb, colmn, ncol,
-                                                                         q0, qc, n, (__nv_bfloat16*)out);
-  else if (mode == 5)
-    df_unpack_kernel<__nv_bfloat16, float><<<grid, 256, 0, st>>>((const float*)B, ldb, colmn, ncol, q0, qc, n,
-                                                                  (__nv_bfloat16*)out);
-  else if (mode == 3)
-    df_unpack_kernel<double, float><<<grid, 256, 0, st>>>((const float*)B, ldb, colmn, ncol, q0, qc, n, (double*)out);
-  else
-    df_unpack_kernel<double, __nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)B, ldb, colmn, ncol, q0, qc,
-                                                                  n, (double*)out);
-  return cudaGetLastError();
+cudaError_t launch_df_unpack(int mode, const void* B, long long ldb, const int* map, int q0, int qc, int n, void* out,
+                             cudaStream_t st) {
+  if (qc <= 0) return cudaSuccess;
+  // about 32 Q per block, so that the map is read once per 32 elements
+  const dim3 grid((unsigned)((n + 63) / 64), (unsigned)((n + 3) / 4), (unsigned)std::min(qc, std::max(1, (qc + 31) / 32)));
+  auto run = [&](auto kern, auto* src, auto* dst) {
+    kern<<<grid, 256, 0, st>>>(src, ldb, map, q0, qc, n, dst);
+    return cudaGetLastError();
+  };
+  using bf = __nv_bfloat16;
+  if (mode == 0) return run(df_unpack_kernel<double, double>, (const double*)B, (double*)out);
+  if (mode == 1) return run(df_unpack_kernel<float, float>, (const float*)B, (float*)out);
+  if (mode == 2) return run(df_unpack_kernel<bf, bf>, (const bf*)B, (bf*)out);
+  if (mode == 5) return run(df_unpack_kernel<bf, float>, (const float*)B, (bf*)out);
+  if (mode == 3) return run(df_unpack_kernel<double, float>, (const float*)B, (double*)out);
+  return run(df_unpack_kernel<double, bf>, (const bf*)B, (double*)out);
 }
 
 // J contractions on a stored FP32 / BF16 factor with FP64 accumulation

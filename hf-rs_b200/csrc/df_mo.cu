@@ -7,12 +7,16 @@
 //   mp2_energy: E = sum_{ij in active occ, ab in virt} v_iajb (2 v_iajb - v_ibja)
 //              / (e_i + e_j - e_a - e_b), v_iajb = sum_Q B_Q,ia B_Q,jb.
 // FP64 throughout, on the stored factor (FP32 / BF16 storage converted while
-// unpacking).  Per chunk of Q: unpack B_Q dense, T_Q = C^T B_Q and
-// M_Q = T_Q C by batched cuBLAS DGEMMs (plain library GEMMs), then either
-// pack M_Q or keep its occupied-virtual block L[Q][i][a].  The MP2 energy is
-// one DGEMM per active occupied i, V_i[a][(j, b)] = sum_Q L[Q][i][a] L[Q][j][b],
-// and a reduction kernel that applies the denominators (this library's own,
-// one partial sum per block, summed on the host in a fixed order).
+// unpacking).  Per chunk of Q: unpack B_Q dense; the transform then forms
+// T_Q = C^T B_Q and M_Q = T_Q C by batched cuBLAS DGEMMs (plain library
+// GEMMs) and packs M_Q.  MP2 needs the occupied-virtual block
+// L[Q][i][a] only: U = B_Q C_occ for the whole chunk in one GEMM, then
+// L_Q = C_virt^T U_Q, (n_occ / m)(1 + n_virt / m) of the full transform's
+// work or less.  The energy takes blocks of occupied orbitals i against
+// every j up to the block's last, V[(i, a)][(j, b)] = sum_Q L[Q][i][a]
+// L[Q][j][b] (the pair (j, i) equals (i, j)), and a reduction kernel that
+// applies the denominators (this library's own; its partial sums come to the
+// host once and are added in a fixed order).
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
@@ -43,57 +47,56 @@ __global__ void pack_mo_kernel(const double* __restrict__ M, int m, int qn, doub
   }
 }
 
-// L[q][i][a] = M[q][o0 + i][v0 + a] for the occupied-virtual block
-__global__ void ov_block_kernel(const double* __restrict__ M, int m, int qn, int o0, int no, int v0, int nv,
-                                double* __restrict__ L) {
-  const long long tot = (long long)qn * no * nv;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(t / ((long long)no * nv));
-    const int r = (int)(t % ((long long)no * nv));
-    const int i = r / nv, a = r % nv;
-    L[t] = M[(size_t)q * m * m + (size_t)(o0 + i) * m + v0 + a];
-  }
-}
-
-// Energy of one occupied i: V is (j, b, a) with V[(j * nv + b) * nv + a] =
-// v_iajb.  Each block writes one partial sum.
-__global__ void mp2_pair_kernel(const double* __restrict__ V, const double* __restrict__ eps, int i, int o0, int no,
-                                int v0, int nv, double* __restrict__ part) {
+// Energy of the pairs (i, j <= i) of a block of ni occupied orbitals from i0
+// (of the active ones): V[(j nv + b) ld + i nv + a] = v_iajb with i counted
+// from i0, ld = ni nv; pairs with j < i count twice.  One block of threads
+// per (i, b range); each writes one partial sum.
+__global__ void __launch_bounds__(256) mp2_pair_kernel(const double* __restrict__ V, const double* __restrict__ eps,
+                                                       int i0, int ni, int o0, int v0, int nv,
+                                                       double* __restrict__ part) {
   double s = 0.0;
-  const long long tot = (long long)no * nv * nv;
+  const size_t ld = (size_t)ni * nv;
+  const int il = blockIdx.y, i = i0 + il;
   const double ei = eps[o0 + i];
+  const long long tot = (long long)(i + 1) * nv * nv;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(t / ((long long)nv * nv));
     const int r = (int)(t % ((long long)nv * nv));
     const int b = r / nv, a = r % nv;
-    const double v = V[t];                                   // v_iajb
-    const double w = V[((size_t)j * nv + a) * nv + b];        // v_ibja
+    const double v = V[((size_t)j * nv + b) * ld + (size_t)il * nv + a];  // v_iajb
+    const double w = V[((size_t)j * nv + a) * ld + (size_t)il * nv + b];  // v_ibja
     const double gap = ei + eps[o0 + j] - eps[v0 + a] - eps[v0 + b];
-    s += v * (2.0 * v - w) / gap;
+    const double e = v * (2.0 * v - w) / gap;
+    s += j < i ? 2.0 * e : e;
   }
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  __shared__ double w32[32];
+  __shared__ double w32[8];
   if ((threadIdx.x & 31) == 0) w32[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += w32[k];
-    part[blockIdx.x] = t;
+    part[blockIdx.y * gridDim.x + blockIdx.x] = t;
   }
+}
+
+// The chunk's rows [q0, q0 + qn) of the factor, dense (interleaved
+// [row][q][col], as launch_df_unpack lays them out).
+int unpack_chunk(hfg_df* df, int q0, int qn, double* dense) {
+  hfg_ctx* ctx = df->ctx;
+  const int rc = df->ensure_map();
+  if (rc != HFG_OK) return rc;
+  const int um = df->storage == HFG_DF_FP64 ? 0 : (df->storage == HFG_DF_FP32 ? 3 : 4);
+  const void* Bs = df->storage == HFG_DF_FP64 ? (const void*)df->B64.p
+                   : df->storage == HFG_DF_FP32 ? (const void*)df->B32.p : (const void*)df->B16.p;
+  return cuda_check(ctx, launch_df_unpack(um, Bs, df->ncol, df->map.p, q0, qn, df->n, dense, ctx->stream), "unpack");
 }
 
 // M_Q = C^T B_Q C for the chunk [q0, q0 + qn): C row-major n x m on the device.
 int mo_chunk(hfg_df* df, const double* dC, int m, int q0, int qn, double* dense, double* T, double* M) {
   hfg_ctx* ctx = df->ctx;
-  cudaStream_t st = ctx->stream;
   const int n = df->n;
-  const long long nn = (long long)n * n;
-  int rc = cuda_check(ctx, cudaMemsetAsync(dense, 0, (size_t)qn * nn * 8, st), "clear");
-  if (rc != HFG_OK) return rc;
-  const int um = df->storage == HFG_DF_FP64 ? 0 : (df->storage == HFG_DF_FP32 ? 3 : 4);
-  const void* Bs = df->storage == HFG_DF_FP64 ? (const void*)df->B64.p
-                   : df->storage == HFG_DF_FP32 ? (const void*)df->B32.p : (const void*)df->B16.p;
-  rc = cuda_check(ctx, launch_df_unpack(um, Bs, df->ncol, df->colmn.p, df->ncol, q0, qn, n, dense, st), "unpack");
+  const int rc = unpack_chunk(df, q0, qn, dense);
   if (rc != HFG_OK) return rc;
   const double one = 1.0, zero = 0.0;
   // column-major views: C row-major (n x m) is Cc = C^T (m x n, ld m); the
@@ -109,11 +112,12 @@ int mo_chunk(hfg_df* df, const double* dC, int m, int q0, int qn, double* dense,
   return HFG_OK;
 }
 
-int chunk_size(const hfg_df* df, int m) {
+// Q per chunk when each needs n^2 + extra doubles of scratch.
+int chunk_size(const hfg_df* df, size_t extra) {
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const size_t budget = std::max<size_t>((size_t)64 << 20, std::min<size_t>((size_t)4 << 30, free_b / 4));
-  const size_t per_q = ((size_t)df->n * df->n + (size_t)m * df->n + (size_t)m * m) * 8;
+  const size_t per_q = ((size_t)df->n * df->n + extra) * 8;
   return (int)std::max<size_t>(1, std::min<size_t>((size_t)df->rank, budget / per_q));
 }
 
@@ -131,7 +135,7 @@ extern "C" int hfg_df_transform(hfg_df* df, const double* C, int m, double* out,
   cudaSetDevice(ctx->device);
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t st = ctx->stream;
-  const int n = df->n, qc = chunk_size(df, m);
+  const int n = df->n, qc = chunk_size(df, (size_t)m * n + (size_t)m * m);
   DevBuf<double> dC, dense, T, M, P;
   int rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dense.alloc((size_t)qc * n * n), "alloc");
@@ -185,44 +189,56 @@ extern "C" int hfg_df_mp2(hfg_df* df, const double* C, const double* eps, int m,
   cudaSetDevice(ctx->device);
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t st = ctx->stream;
-  const int n = df->n, qc = chunk_size(df, m), rank = df->rank;
-  DevBuf<double> dC, dE, dense, T, M, L, V, part;
-  constexpr int kBlocks = 296;
+  const int n = df->n, qc = chunk_size(df, (size_t)n * no), rank = df->rank;
+  // occupied orbitals per block: about 768 rows of V, so that a block's GEMM
+  // fills the GPU while the block's own upper triangle of pairs (computed
+  // for nothing) stays small
+  const int ib = std::max(1, std::min(no, 768 / nv));
+  const int nblk = (no + ib - 1) / ib;
+  constexpr int kParts = 32;  // partial sums per occupied orbital
+  DevBuf<double> dC, dE, dense, U, L, V, part;
   int rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dE.alloc(m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dense.alloc((size_t)qc * n * n), "alloc");
-  if (rc == HFG_OK) rc = cuda_check(ctx, T.alloc((size_t)qc * m * n), "alloc");
-  if (rc == HFG_OK) rc = cuda_check(ctx, M.alloc((size_t)qc * m * m), "alloc");
+  if (rc == HFG_OK) rc = cuda_check(ctx, U.alloc((size_t)qc * n * no), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, L.alloc((size_t)rank * no * nv), "alloc (ia|Q) factor");
-  if (rc == HFG_OK) rc = cuda_check(ctx, V.alloc((size_t)nv * no * nv), "alloc");
-  if (rc == HFG_OK) rc = cuda_check(ctx, part.alloc(kBlocks), "alloc");
+  if (rc == HFG_OK) rc = cuda_check(ctx, V.alloc((size_t)ib * nv * no * nv), "alloc");
+  if (rc == HFG_OK) rc = cuda_check(ctx, part.alloc((size_t)kParts * no), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, cudaMemcpyAsync(dC.p, C, (size_t)n * m * 8, cudaMemcpyHostToDevice, st), "copy C");
   if (rc == HFG_OK) rc = cuda_check(ctx, cudaMemcpyAsync(dE.p, eps, (size_t)m * 8, cudaMemcpyHostToDevice, st), "copy eps");
   if (rc != HFG_OK) return rc;
+  const double one = 1.0, zero = 0.0;
   for (int q0 = 0; q0 < rank; q0 += qc) {
     const int qn = std::min(qc, rank - q0);
-    rc = mo_chunk(df, dC.p, m, q0, qn, dense.p, T.p, M.p);
+    rc = unpack_chunk(df, q0, qn, dense.p);
     if (rc != HFG_OK) return rc;
-    ov_block_kernel<<<1184, 256, 0, st>>>(M.p, m, qn, n_frozen, no, n_occ, nv, L.p + (size_t)q0 * no * nv);
-    rc = cuda_check(ctx, cudaGetLastError(), "occupied-virtual block");
-    if (rc != HFG_OK) return rc;
+    // column-major views: the dense chunk is X ((q, k) x row, ld qn n) and C
+    // row-major (n x m) is Cc = C^T (m x n, ld m).  U = X C_occ, then
+    // L_Q (nv x no) = C_virt^T U_Q
+    if (cublasDgemm(df->blas, CUBLAS_OP_N, CUBLAS_OP_T, qn * n, no, n, &one, dense.p, qn * n, dC.p + n_frozen, m, &zero,
+                    U.p, qn * n) != CUBLAS_STATUS_SUCCESS ||
+        cublasDgemmStridedBatched(df->blas, CUBLAS_OP_N, CUBLAS_OP_N, nv, no, n, &one, dC.p + n_occ, m, 0, U.p, qn * n, n,
+                                  &zero, L.p + (size_t)q0 * no * nv, nv, (long long)no * nv, qn) != CUBLAS_STATUS_SUCCESS)
+      return set_error(ctx, HFG_ERR_CUDA, "RI-MP2 transform GEMM");
   }
-  const double one = 1.0, zero = 0.0;
   const int ld = no * nv;
-  std::vector<double> h(kBlocks);
-  double e = 0.0;
-  for (int i = 0; i < no; ++i) {
-    // V[a][(j, b)] = sum_Q L[Q][i][a] L[Q][j][b]
-    if (cublasDgemm(df->blas, CUBLAS_OP_N, CUBLAS_OP_T, nv, no * nv, rank, &one, L.p + (size_t)i * nv, ld, L.p, ld,
-                    &zero, V.p, nv) != CUBLAS_STATUS_SUCCESS)
+  for (int k = 0; k < nblk; ++k) {
+    const int i0 = k * ib, ni = std::min(ib, no - i0), nj = i0 + ni;
+    // V[(i, a)][(j, b)] = sum_Q L[Q][i][a] L[Q][j][b], j < nj
+    if (cublasDgemm(df->blas, CUBLAS_OP_N, CUBLAS_OP_T, ni * nv, nj * nv, rank, &one, L.p + (size_t)i0 * nv, ld, L.p, ld,
+                    &zero, V.p, ni * nv) != CUBLAS_STATUS_SUCCESS)
       return set_error(ctx, HFG_ERR_CUDA, "RI-MP2 GEMM");
-    mp2_pair_kernel<<<kBlocks, 256, 0, st>>>(V.p, dE.p, i, n_frozen, no, n_occ, nv, part.p);
+    mp2_pair_kernel<<<dim3(kParts, (unsigned)ni), 256, 0, st>>>(V.p, dE.p, i0, ni, n_frozen, n_occ, nv,
+                                                                part.p + (size_t)i0 * kParts);
     rc = cuda_check(ctx, cudaGetLastError(), "RI-MP2 energy");
-    if (rc == HFG_OK) rc = cuda_check(ctx, cudaMemcpyAsync(h.data(), part.p, kBlocks * 8, cudaMemcpyDeviceToHost, st), "copy");
-    if (rc == HFG_OK) rc = cuda_check(ctx, cudaStreamSynchronize(st), "RI-MP2");
     if (rc != HFG_OK) return rc;
-    for (double x : h) e += x;
   }
+  std::vector<double> h((size_t)kParts * no);
+  rc = cuda_check(ctx, cudaMemcpyAsync(h.data(), part.p, h.size() * 8, cudaMemcpyDeviceToHost, st), "copy");
+  if (rc == HFG_OK) rc = cuda_check(ctx, cudaStreamSynchronize(st), "RI-MP2");
+  if (rc != HFG_OK) return rc;
+  double e = 0.0;
+  for (double x : h) e += x;
   *energy = e;
   return HFG_OK;
 }

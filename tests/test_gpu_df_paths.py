@@ -33,3 +33,30 @@ def test_tensor_core_exchange_over_occupied_counts(cluster, nocc, mma, tol):
     assert np.max(np.abs(J - J0)) <= 1e-12 * np.max(np.abs(J0))
     assert np.linalg.norm(K - K0) < tol * np.linalg.norm(K0)
     assert np.array_equal(K, K.T)
+
+
+@pytest.mark.parametrize("n_occ,frozen", [(1, 0), (10, 0), (10, 3), (33, 1), (49, 0)])
+@pytest.mark.parametrize("storage", [HFG_DF_FP64, HFG_DF_FP32])
+def test_ri_mp2_matches_its_definition_on_the_transformed_factor(n_occ, frozen, storage):
+    # blocks of 15 to 768 occupied orbitals, whole and ragged
+    atoms = water_cluster(2)
+    ctx = Context(CartesianBasis.build(atoms, "cc-pvdz"))
+    df = DFTensor(ctx, CartesianBasis.build(atoms, AUX), storage=storage)
+    n = ctx.n
+    rng = np.random.default_rng(n_occ)
+    C = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    eps = np.concatenate([np.sort(rng.uniform(-3, -0.5, n_occ)), np.sort(rng.uniform(0.3, 3, n - n_occ))])
+    B = np.zeros((df.sizes()[1], n, n))
+    i, j = np.tril_indices(n)
+    B[:, i, j] = df.transform(C)
+    B[:, j, i] = B[:, i, j]
+    L = B[:, frozen:n_occ, n_occ:]
+    v = np.einsum("qia,qjb->iajb", L, L, optimize=True)
+    eo, ev = eps[frozen:n_occ], eps[n_occ:]
+    gap = eo[:, None, None, None] - ev[None, :, None, None] + eo[None, None, :, None] - ev[None, None, None, :]
+    want = np.sum(v * (2.0 * v - v.transpose(0, 3, 2, 1)) / gap)
+    got = df.mp2_energy(C, eps, n_occ, frozen)
+    # n_occ^2 n_virt^2 products of 64-bit sums over ~260 functions
+    assert abs(got - want) < 1e-11 * abs(want)
+    df.close()
+    ctx.close()
