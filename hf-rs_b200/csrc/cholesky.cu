@@ -263,8 +263,6 @@ extern "C" int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, h
   df->n = (int)n;
   df->storage = HFG_DF_FP64;
   CK(df->B64.alloc((size_t)cap * np));
-  if (cublasCreate(&df->blas) != CUBLAS_STATUS_SUCCESS) return set_error(ctx, HFG_ERR_CUDA, "cublasCreate");
-  cublasSetStream(df->blas, st);
   std::vector<long long> piv;
   long long rank = 0;
   double maxres = 0.0;

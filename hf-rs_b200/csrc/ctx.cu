@@ -971,6 +971,7 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
 }  // namespace hfg
 
 hfg_ctx::~hfg_ctx() {
+  if (free_handles) free_handles(this);
   for (auto* map : {&plans, &other_plans[0], &other_plans[1], &other_plans[2]})
     for (auto& kv : *map)
       for (auto& L : kv.second->launches) {

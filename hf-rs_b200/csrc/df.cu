@@ -92,6 +92,63 @@ int make_aux_set(hfg_ctx* ctx, const hfg_basis* aux, AuxSet& ax) {
   return cuda_check(ctx, cudaStreamSynchronize(st), "aux set");
 }
 
+// The three-centre launches of one set of columns: every bra class against
+// every auxiliary angular momentum, over the context stream and its side
+// streams, with the classes' index lists in one upload.
+struct Launch3c {
+  struct Bra {
+    int la, lb, n;
+    size_t off;
+    const PairInfo* pairs;
+    const PrimPair* prims;
+    double mean;  // primitive pairs per pair
+  };
+  hfg_ctx* ctx;
+  std::vector<Bra> bras;
+  std::vector<int> idx;
+  std::vector<long long> col;
+  explicit Launch3c(hfg_ctx* c) : ctx(c) {}
+  void add(int la, int lb, const PairInfo* pairs, const PrimPair* prims, double mean, const std::vector<int>& i,
+           const std::vector<long long>& c) {
+    bras.push_back({la, lb, (int)i.size(), idx.size(), pairs, prims, mean});
+    idx.insert(idx.end(), i.begin(), i.end());
+    col.insert(col.end(), c.begin(), c.end());
+  }
+  // out[aux function][column] with leading dimension ld
+  int run(AuxSet& ax, double* out, long long ld) {
+    cudaStream_t st = ctx->stream;
+    DevBuf<int> didx;
+    DevBuf<long long> dcol;
+    int rc = cuda_check(ctx, didx.alloc(idx.size()), "alloc");
+    if (rc == HFG_OK) rc = cuda_check(ctx, dcol.alloc(col.size()), "alloc");
+    if (rc == HFG_OK)
+      rc = cuda_check(ctx, cudaMemcpyAsync(didx.p, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, st), "copy");
+    if (rc == HFG_OK)
+      rc = cuda_check(ctx, cudaMemcpyAsync(dcol.p, col.data(), col.size() * 8, cudaMemcpyHostToDevice, st), "copy");
+    if (rc == HFG_OK) rc = cuda_check(ctx, ctx->ensure_side_streams(), "side streams");
+    if (rc == HFG_OK) rc = cuda_check(ctx, cudaEventRecord(ctx->ev_fork, st), "fork");
+    if (rc != HFG_OK) return rc;
+    for (auto& s : ctx->side) cudaStreamWaitEvent(s, ctx->ev_fork, 0);
+    int launch = 0;
+    // the heavy classes first
+    for (auto b = bras.rbegin(); b != bras.rend(); ++b)
+      for (auto kk = ax.by_l.rbegin(); kk != ax.by_l.rend() && rc == HFG_OK; ++kk) {
+        const Df3cArgs a{b->pairs, b->prims, didx.p + b->off, dcol.p + b->off, b->n, ax.dup.p, ax.dupr.p,
+                         ax.idx[kk->first].p, (int)kk->second.size(), ctx->d_boys64.p, ctx->d_expt64.p, out, ld, 1,
+                         b->mean};
+        const int si = launch++ % (1 + kJKSideStreams);
+        rc = cuda_check(ctx, launch_df3c(b->la, b->lb, kk->first, a, si == 0 ? st : ctx->side[si - 1]),
+                        "three-centre kernel");
+      }
+    // joined on every path: the lists are released in the context stream's order
+    for (int k = 0; k < kJKSideStreams; ++k) {
+      cudaEventRecord(ctx->ev_join[k], ctx->side[k]);
+      cudaStreamWaitEvent(st, ctx->ev_join[k], 0);
+    }
+    return rc;
+  }
+};
+
 int gemm_ex(hfg_ctx* ctx, cublasHandle_t h, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k,
             const void* A, cudaDataType ta_t, int lda, const void* B, cudaDataType tb_t, int ldb, float beta,
             float* C, int ldc, cublasComputeType_t ct) {
@@ -172,26 +229,22 @@ int hfg_df_build_shard(hfg_ctx* ctx, const hfg_basis* aux, double metric_cutoff,
   DevBuf<PairInfo>& dup = ax.dup;
   DevBuf<PrimPair>& dupr = ax.dupr;
   std::map<int, std::vector<int>>& aux_by_l = ax.by_l;
-  std::map<int, DevBuf<int>>& aux_idx = ax.idx;
   // metric (P|Q): bra and ket both unit-paired auxiliary shells
   CK(df->metric.alloc((size_t)naux * naux));
-  for (auto& bk : aux_by_l) {
-    std::vector<long long> cols;
-    for (int s : bk.second) cols.push_back(auxc.shells[s].ao);
-    DevBuf<long long> dcols;
-    CK(dcols.alloc(cols.size()));
-    CK(cudaMemcpyAsync(dcols.p, cols.data(), cols.size() * 8, cudaMemcpyHostToDevice, st));
-    for (auto& kk : aux_by_l) {
-      Df3cArgs a{dup.p, dupr.p, aux_idx[bk.first].p, dcols.p, (int)bk.second.size(), dup.p, dupr.p,
-                 aux_idx[kk.first].p, (int)kk.second.size(), ctx->d_boys64.p, ctx->d_expt64.p, df->metric.p, naux};
-      CK(launch_df3c(bk.first, 0, kk.first, a, st));
+  {
+    Launch3c l3(ctx);
+    for (auto& bk : aux_by_l) {
+      std::vector<long long> cols;
+      for (int s : bk.second) cols.push_back(auxc.shells[s].ao);
+      l3.add(bk.first, 0, dup.p, dupr.p, 1.0, bk.second, cols);
     }
-    CK(cudaStreamSynchronize(st));
+    rc = l3.run(ax, df->metric.p, naux);
+    if (rc != HFG_OK) return rc;
   }
   // canonical orthogonaliser of the metric (cutoff on its eigenvalues)
   cusolverDnHandle_t solver = nullptr;
-  if (cusolverDnCreate(&solver) != CUSOLVER_STATUS_SUCCESS) return set_error(ctx, HFG_ERR_CUDA, "cusolver");
-  cusolverDnSetStream(solver, st);
+  rc = ctx_handles(ctx, &df->blas, &solver);
+  if (rc != HFG_OK) return rc;
   DevBuf<double> V, w, work;
   DevBuf<int> info;
   CK(V.alloc((size_t)naux * naux));
@@ -202,14 +255,11 @@ int hfg_df_build_shard(hfg_ctx* ctx, const hfg_basis* aux, double metric_cutoff,
   cusolverDnDsyevd_bufferSize(solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, naux, V.p, naux, w.p, &lwork);
   CK(work.alloc(lwork));
   if (cusolverDnDsyevd(solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, naux, V.p, naux, w.p, work.p, lwork,
-                       info.p) != CUSOLVER_STATUS_SUCCESS) {
-    cusolverDnDestroy(solver);
+                       info.p) != CUSOLVER_STATUS_SUCCESS)
     return set_error(ctx, HFG_ERR_CUDA, "metric eigendecomposition failed");
-  }
   std::vector<double> wh(naux);
   CK(cudaMemcpyAsync(wh.data(), w.p, naux * 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  cusolverDnDestroy(solver);
   if (wh[0] < -metric_cutoff) return set_error(ctx, HFG_ERR_INTEGRAL, "DF metric has a negative eigenvalue");
   int first = 0;
   while (first < naux && wh[first] < metric_cutoff) ++first;
@@ -223,17 +273,9 @@ int hfg_df_build_shard(hfg_ctx* ctx, const hfg_basis* aux, double metric_cutoff,
   df->rank_total = rank_total;
   df->row0 = row0;
   // Xm = V[:, first + row0 : first + row0 + rank] diag(w^-1/2), column-major
-  // naux x rank (columns move left only, so none is overwritten before use)
-  {
-    std::vector<double> Vh((size_t)naux * naux);
-    CK(cudaMemcpyAsync(Vh.data(), V.p, Vh.size() * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (int c = 0; c < rank; ++c) {
-      const double sc = 1.0 / std::sqrt(wh[first + row0 + c]);
-      for (int r = 0; r < naux; ++r) Vh[(size_t)c * naux + r] = Vh[(size_t)(first + row0 + c) * naux + r] * sc;
-    }
-    CK(cudaMemcpyAsync(V.p, Vh.data(), (size_t)naux * rank * 8, cudaMemcpyHostToDevice, st));
-  }
+  // naux x rank, scaled in place
+  double* const Xm = V.p + (size_t)(first + row0) * naux;
+  CK(launch_whiten(Xm, w.p + first + row0, naux, rank, st));
 
   // significant orbital shell pairs (in pair order) and their unique AO-pair columns
   struct SigPair {
@@ -259,8 +301,6 @@ int hfg_df_build_shard(hfg_ctx* ctx, const hfg_basis* aux, double metric_cutoff,
   df->ncol = ncol;
   CK(df->colmn.alloc(ncol));
   CK(cudaMemcpyAsync(df->colmn.p, colmn.data(), ncol * sizeof(int2), cudaMemcpyHostToDevice, st));
-  if (cublasCreate(&df->blas) != CUBLAS_STATUS_SUCCESS) return set_error(ctx, HFG_ERR_CUDA, "cublasCreate");
-  cublasSetStream(df->blas, st);
   // the stored factor B (row-major [rank][ncol]) in its storage precision
   if (storage == HFG_DF_FP64) CK(df->B64.alloc((size_t)rank * ncol));
   else if (storage == HFG_DF_FP32) CK(df->B32.alloc((size_t)rank * ncol));
@@ -297,26 +337,21 @@ int hfg_df_build_shard(hfg_ctx* ctx, const hfg_basis* aux, double metric_cutoff,
       e.first.push_back(sig[k].pair);
       e.second.push_back(sig[k].col - c0);
     }
+    Launch3c l3(ctx);
     for (auto& bc : by_class) {
-      DevBuf<int> bidx;
-      DevBuf<long long> bcol;
-      CK(bidx.alloc(bc.second.first.size()));
-      CK(bcol.alloc(bc.second.second.size()));
-      CK(cudaMemcpyAsync(bidx.p, bc.second.first.data(), bc.second.first.size() * 4, cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(bcol.p, bc.second.second.data(), bc.second.second.size() * 8, cudaMemcpyHostToDevice, st));
-      for (auto& kk : aux_by_l) {
-        Df3cArgs a{ctx->d_pairs.p, ctx->d_prims.p, bidx.p, bcol.p, (int)bc.second.first.size(), dup.p, dupr.p,
-                   aux_idx[kk.first].p, (int)kk.second.size(), ctx->d_boys64.p, ctx->d_expt64.p, T3.p, w};
-        CK(launch_df3c(bc.first.first, bc.first.second, kk.first, a, st));
-      }
-      CK(cudaStreamSynchronize(st));  // the index buffers are released at the end of this scope
+      double prims = 0.0;
+      for (int p : bc.second.first) prims += ctx->h_pairs[p].npp;
+      l3.add(bc.first.first, bc.first.second, ctx->d_pairs.p, ctx->d_prims.p, prims / (double)bc.second.first.size(),
+             bc.second.first, bc.second.second);
     }
+    rc = l3.run(ax, T3.p, w);
+    if (rc != HFG_OK) return rc;
     // column-major view: T3c (w x naux, ld w) times Xm (naux x rank) gives the
     // chunk's columns of B (row-major [rank][ncol] = column-major ncol x rank)
     const double one = 1.0, zero = 0.0;
     double* dst = storage == HFG_DF_FP64 ? df->B64.p + c0 : Bt.p;
     const int ldc = storage == HFG_DF_FP64 ? (int)ncol : w;
-    if (cublasDgemm(df->blas, CUBLAS_OP_N, CUBLAS_OP_N, w, rank, naux, &one, T3.p, w, V.p, naux, &zero, dst, ldc) !=
+    if (cublasDgemm(df->blas, CUBLAS_OP_N, CUBLAS_OP_N, w, rank, naux, &one, T3.p, w, Xm, naux, &zero, dst, ldc) !=
         CUBLAS_STATUS_SUCCESS)
       return set_error(ctx, HFG_ERR_CUDA, "B = X^T (P|mn) GEMM failed");
     if (storage != HFG_DF_FP64)
@@ -413,24 +448,15 @@ int hfg_df_three_center(hfg_ctx* ctx, const hfg_basis* aux, double* out, size_t 
   DevBuf<double> T3;
   rc = cuda_check(ctx, T3.alloc((size_t)naux * ncol), "alloc three-centre");
   if (rc != HFG_OK) return rc;
-  for (auto& bc : by_class) {
-    DevBuf<int> bidx;
-    DevBuf<long long> bcol;
-    rc = cuda_check(ctx, bidx.alloc(bc.second.first.size()), "alloc");
-    if (rc == HFG_OK) rc = cuda_check(ctx, bcol.alloc(bc.second.second.size()), "alloc");
-    if (rc == HFG_OK)
-      rc = cuda_check(ctx, cudaMemcpyAsync(bidx.p, bc.second.first.data(), bc.second.first.size() * 4,
-                                           cudaMemcpyHostToDevice, st), "copy");
-    if (rc == HFG_OK)
-      rc = cuda_check(ctx, cudaMemcpyAsync(bcol.p, bc.second.second.data(), bc.second.second.size() * 8,
-                                           cudaMemcpyHostToDevice, st), "copy");
-    for (auto& kk : ax.by_l) {
-      if (rc != HFG_OK) break;
-      Df3cArgs a{ctx->d_pairs.p, ctx->d_prims.p, bidx.p, bcol.p, (int)bc.second.first.size(), ax.dup.p, ax.dupr.p,
-                 ax.idx[kk.first].p, (int)kk.second.size(), ctx->d_boys64.p, ctx->d_expt64.p, T3.p, ncol};
-      rc = cuda_check(ctx, launch_df3c(bc.first.first, bc.first.second, kk.first, a, st), "three-centre kernel");
+  {
+    Launch3c l3(ctx);
+    for (auto& bc : by_class) {
+      double prims = 0.0;
+      for (int p : bc.second.first) prims += ctx->h_pairs[p].npp;
+      l3.add(bc.first.first, bc.first.second, ctx->d_pairs.p, ctx->d_prims.p, prims / (double)bc.second.first.size(),
+             bc.second.first, bc.second.second);
     }
-    if (rc == HFG_OK) rc = cuda_check(ctx, cudaStreamSynchronize(st), "three-centre");
+    rc = l3.run(ax, T3.p, ncol);
     if (rc != HFG_OK) return rc;
   }
   std::vector<double> h((size_t)naux * ncol);
@@ -457,6 +483,28 @@ int hfg_df::ensure_map() {
 
 namespace hfg {
 
+int ctx_handles(hfg_ctx* ctx, cublasHandle_t* blas, cusolverDnHandle_t* solver) {
+  ctx->free_handles = [](hfg_ctx* c) {
+    if (c->blas) cublasDestroy((cublasHandle_t)c->blas);
+    if (c->solver) cusolverDnDestroy((cusolverDnHandle_t)c->solver);
+  };
+  if (blas && !ctx->blas) {
+    cublasHandle_t h = nullptr;
+    if (cublasCreate(&h) != CUBLAS_STATUS_SUCCESS) return set_error(ctx, HFG_ERR_CUDA, "cublasCreate");
+    ctx->blas = h;
+    cublasSetStream(h, ctx->stream);
+  }
+  if (solver && !ctx->solver) {
+    cusolverDnHandle_t h = nullptr;
+    if (cusolverDnCreate(&h) != CUSOLVER_STATUS_SUCCESS) return set_error(ctx, HFG_ERR_CUDA, "cusolver");
+    ctx->solver = h;
+    cusolverDnSetStream(h, ctx->stream);
+  }
+  if (blas) *blas = (cublasHandle_t)ctx->blas;
+  if (solver) *solver = (cusolverDnHandle_t)ctx->solver;
+  return HFG_OK;
+}
+
 bool df_is_shard(const hfg_df* df) { return df->shard(); }
 
 // J and K from occupied coefficients on the device: dC column-major n x nocc
@@ -470,7 +518,8 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
   if (q_lo < 0 || q_lo > q_hi || q_hi > df->rank) return set_error(ctx, HFG_ERR_INVALID_INPUT, "auxiliary range");
   const int rank = q_hi - q_lo;
   const long long ncol = df->ncol, nn = (long long)n * n;
-  int rc = HFG_OK;
+  int rc = df->bind();
+  if (rc != HFG_OK) return rc;
 #define CK(call)                         \
   do {                                   \
     rc = cuda_check(ctx, (call), #call); \

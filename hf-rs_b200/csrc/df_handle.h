@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "df_umma.h"
+#include "handles.h"
 #include "hfg_ctx.h"
 
 // B = X^T (P|mn) over the stored AO pairs, row-major [rank][ncol], in its
@@ -25,7 +26,8 @@ struct hfg_df {
   // (in hfg_df's context, lock held)
   int ensure_map();
   hfg::DevBuf<double> metric;  // kept for inspection (naux x naux)
-  cublasHandle_t blas = nullptr;
+  cublasHandle_t blas = nullptr;  // the context's, set by bind() in every entry point
+  int bind() { return hfg::ctx_handles(ctx, &blas, nullptr); }
   hfg::DevBuf<double> P, pvec, gam, jcol, Cd, J, K, T64;
   hfg::DevBuf<float> gam32, jcol32, pvec32, Kf, Tf, Cf;
   hfg::DevBuf<__nv_bfloat16> Cb, Tb;
@@ -44,6 +46,5 @@ struct hfg_df {
   ~hfg_df() {
     for (auto& e : kev)
       if (e) cudaEventDestroy(e);
-    if (blas) cublasDestroy(blas);
   }
 };

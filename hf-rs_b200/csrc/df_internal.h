@@ -20,12 +20,17 @@ struct Df3cArgs {
   const double* expt;
   double* out;  // out[aux function][column], leading dimension ld
   long long ld;
+  int lanes;    // lanes per (bra, ket) combination (a power of two; launch_df3c chooses)
+  double prims; // mean primitive pairs of the bra pairs
 };
 
-cudaError_t launch_df3c(int la, int lb, int lc, const Df3cArgs& args, cudaStream_t st);
+cudaError_t launch_df3c(int la, int lb, int lc, Df3cArgs args, cudaStream_t st);
+// The same on the block-per-quartet engine (eri_md.cu).
+cudaError_t launch_df3c_md(int la, int lb, int lc, const Df3cArgs& args, cudaStream_t st);
 cudaError_t launch_df_map(const int2* colmn, long long ncol, int n, int* map, cudaStream_t st);
 cudaError_t launch_df_unpack(int mode, const void* B, long long ldb, const int* map, int q0, int qc, int n, void* out,
                              cudaStream_t st);
+cudaError_t launch_whiten(double* X, const double* w, int rows, int cols, cudaStream_t st);
 cudaError_t launch_convert(int mode, const double* in, void* out, long long len, cudaStream_t st);
 cudaError_t launch_convert_cols(int mode, const double* in, int w, long long rows, void* out, long long ldo,
                                 long long c0, cudaStream_t st);

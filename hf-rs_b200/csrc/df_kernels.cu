@@ -52,7 +52,9 @@ __device__ __forceinline__ double comp_scale_any(int l, int i) {
 }
 
 // One block of (ab|P 1): bra pair i (orbital pair or unit-paired auxiliary
-// shell), ket unit pair P.  Thread per (bra, ket) combination of one class.
+// shell), ket unit pair P, by a group of a.lanes lanes that split the bra's
+// primitive pairs and add their accumulators by a butterfly.  Persistent
+// blocks (the Boys table is staged once).
 template <int LA, int LB, int LC>
 __global__ void __launch_bounds__(128) df3c_kernel(const Df3cArgs a) {
   using C = EriClass<LA, LB, LC, 0>;
@@ -61,10 +63,15 @@ __global__ void __launch_bounds__(128) df3c_kernel(const Df3cArgs a) {
   double* sm = reinterpret_cast<double*>(smem_raw);
   boys_stage<double, C::L>(sm, a.boys, a.expt);
   __syncthreads();
-  const long long total = (long long)a.nbra * a.nket;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int ib = (int)(t % a.nbra), ik = (int)(t / a.nbra);
+  const int gs = a.lanes, mem = threadIdx.x & (gs - 1);
+  const long long total = (long long)a.nbra * a.nket, step = (long long)gridDim.x * blockDim.x / gs;
+  const long long t0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / gs;
+  // whole warps go round together (the butterfly needs every lane)
+  for (long long base = 0; base < total; base += step) {
+    const long long t = base + t0;
+    const bool on = t < total;
+    if (__ballot_sync(0xffffffffu, on) == 0u) break;
+    const int ib = on ? (int)(t % a.nbra) : 0, ik = on ? (int)(t / a.nbra) : 0;
     const PairInfo bra = a.bra_pairs[a.bra_idx[ib]];
     const PairInfo ket = a.ket_pairs[a.ket_idx[ik]];
     double acc[C::NACC];
@@ -73,7 +80,7 @@ __global__ void __launch_bounds__(128) df3c_kernel(const Df3cArgs a) {
     const double ACx = bra.Ax - ket.Ax, ACy = bra.Ay - ket.Ay, ACz = bra.Az - ket.Az;
     for (int q = 0; q < ket.npp; ++q) {
       const PrimPair Q = a.ket_prims[ket.pp_off + q];
-      for (int p = 0; p < bra.npp; ++p) {
+      for (int p = mem; p < bra.npp; p += gs) {
         const PrimPair P = a.bra_prims[bra.pp_off + p];
         const double pp = P.p, qq = Q.p;
         const double PQx = ACx + P.PAx - Q.PAx, PQy = ACy + P.PAy - Q.PAy, PQz = ACz + P.PAz - Q.PAz;
@@ -89,6 +96,11 @@ __global__ void __launch_bounds__(128) df3c_kernel(const Df3cArgs a) {
                 ps * PQy, ps * PQz, 0.5 * P.inv_p, 0.5 * Q.inv_p, 0.5 * inv_s, qs, ps);
       }
     }
+    for (int off = 1; off < gs; off <<= 1) {
+#pragma unroll
+      for (int x = 0; x < C::NACC; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], off);
+    }
+    if (!on || mem != 0) continue;
     double out[C::NOUT];
     C::hrr(acc, out, bra.ABx, bra.ABy, bra.ABz, 0.0, 0.0, 0.0);
     // write: rows = ket functions (auxiliary), columns = bra components
@@ -109,21 +121,38 @@ __global__ void __launch_bounds__(128) df3c_kernel(const Df3cArgs a) {
   }
 }
 
-#define HFG_DF_CASE(A, B, Cc)                                                                          \
-  if (la == A && lb == B && lc == Cc) {                                                                \
-    cudaFuncSetAttribute(df3c_kernel<A, B, Cc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);    \
-    df3c_kernel<A, B, Cc><<<grid, 128, smem, st>>>(args);                                              \
-    return cudaGetLastError();                                                                         \
-  }
+template <int LA, int LB, int LC>
+static cudaError_t launch_df3c_class(const Df3cArgs& args, cudaStream_t st) {
+  auto kern = df3c_kernel<LA, LB, LC>;
+  const int smem = (int)boys_smem_bytes<double>();
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
+  const long long want = ((long long)args.nbra * args.nket * args.lanes + 127) / 128,
+                  fit = (long long)sms * (per_sm > 0 ? per_sm : 1);
+  kern<<<(unsigned)std::min(want, fit), 128, smem, st>>>(args);
+  return cudaGetLastError();
+}
+
+#define HFG_DF_CASE(A, B, Cc) \
+  if (la == A && lb == B && lc == Cc) return launch_df3c_class<A, B, Cc>(args, st);
 #define HFG_DF_KETS(A, B) \
   HFG_DF_CASE(A, B, 0) HFG_DF_CASE(A, B, 1) HFG_DF_CASE(A, B, 2) HFG_DF_CASE(A, B, 3) HFG_DF_CASE(A, B, 4)
 
-cudaError_t launch_df3c(int la, int lb, int lc, const Df3cArgs& args, cudaStream_t st) {
+cudaError_t launch_df3c(int la, int lb, int lc, Df3cArgs args, cudaStream_t st) {
   const long long total = (long long)args.nbra * args.nket;
   if (total <= 0) return cudaSuccess;
-  const int smem = (int)boys_smem_bytes<double>();
-  long long g = (total + 127) / 128;
-  const unsigned grid = (unsigned)(g < 148 * 64 ? g : 148 * 64);
+  // the high classes' straight-line code is too long to pass through for few
+  // combinations (factor build and J/K of (H2O)5, 665 auxiliary functions: 15.4
+  // ms with this rule, 17.2 without; 15.3 / 16.6 ms from L = 6 / 4)
+  if (la + lb + lc >= 5 && total <= 20000) return launch_df3c_md(la, lb, lc, args, st);
+  // split the bra's primitive pairs over lanes while there are few
+  // combinations, at least 4 per lane
+  args.lanes = 1;
+  while (args.lanes < 32 && 8 * args.lanes <= args.prims && total * args.lanes < 148 * 1024) args.lanes *= 2;
   HFG_DF_KETS(0, 0)
   HFG_DF_KETS(1, 0)
   HFG_DF_KETS(1, 1)
@@ -259,6 +288,20 @@ __global__ void df_unpack_j_kernel(const double* __restrict__ j, const int2* __r
     J[(long long)mn.x * n + mn.y] = j[c];
     J[(long long)mn.y * n + mn.x] = j[c];
   }
+}
+
+// X[:, c] *= w[c]^{-1/2} (column-major, `rows` rows)
+__global__ void whiten_kernel(double* __restrict__ X, const double* __restrict__ w, int rows, int cols) {
+  const long long len = (long long)rows * cols;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x)
+    X[i] *= 1.0 / sqrt(w[i / rows]);
+}
+
+cudaError_t launch_whiten(double* X, const double* w, int rows, int cols, cudaStream_t st) {
+  const long long len = (long long)rows * cols;
+  if (len <= 0) return cudaSuccess;
+  whiten_kernel<<<(unsigned)std::min<long long>((len + 255) / 256, 148 * 32), 256, 0, st>>>(X, w, rows, cols);
+  return cudaGetLastError();
 }
 
 template <typename TO>

@@ -135,9 +135,11 @@ extern "C" int hfg_df_transform(hfg_df* df, const double* C, int m, double* out,
   cudaSetDevice(ctx->device);
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t st = ctx->stream;
+  int rc = df->bind();
+  if (rc != HFG_OK) return rc;
   const int n = df->n, qc = chunk_size(df, (size_t)m * n + (size_t)m * m);
   DevBuf<double> dC, dense, T, M, P;
-  int rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
+  rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dense.alloc((size_t)qc * n * n), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, T.alloc((size_t)qc * m * n), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, M.alloc((size_t)qc * m * m), "alloc");
@@ -189,6 +191,8 @@ extern "C" int hfg_df_mp2(hfg_df* df, const double* C, const double* eps, int m,
   cudaSetDevice(ctx->device);
   AllocScope alloc_scope(ctx->stream);
   cudaStream_t st = ctx->stream;
+  int rc = df->bind();
+  if (rc != HFG_OK) return rc;
   const int n = df->n, qc = chunk_size(df, (size_t)n * no), rank = df->rank;
   // occupied orbitals per block: about 768 rows of V, so that a block's GEMM
   // fills the GPU while the block's own upper triangle of pairs (computed
@@ -197,7 +201,7 @@ extern "C" int hfg_df_mp2(hfg_df* df, const double* C, const double* eps, int m,
   const int nblk = (no + ib - 1) / ib;
   constexpr int kParts = 32;  // partial sums per occupied orbital
   DevBuf<double> dC, dE, dense, U, L, V, part;
-  int rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
+  rc = cuda_check(ctx, dC.alloc((size_t)n * m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dE.alloc(m), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, dense.alloc((size_t)qc * n * n), "alloc");
   if (rc == HFG_OK) rc = cuda_check(ctx, U.alloc((size_t)qc * n * no), "alloc");

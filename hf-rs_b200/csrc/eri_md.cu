@@ -25,6 +25,7 @@
 
 #include <algorithm>
 
+#include "df_internal.h"
 #include "eri_md.h"
 #include "jk_dispatch.h"
 #include "eri_prim.cuh"
@@ -508,6 +509,33 @@ __global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) 
   }
 }
 
+// Three-centre blocks (ab|P 1) (df_kernels.cu's df3c_kernel) for launches of
+// few combinations in a high class: one combination per block at a time.
+template <int ACC>
+__global__ void __launch_bounds__(ACC == 8 ? 64 : kMDThreads, ACC == 8 ? 8 : 1) df3c_md_kernel(MDClass c, const Df3cArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  MDShared s;
+  md_setup(c, smem_raw, s);
+  const long long total = (long long)a.nbra * a.nket;
+  for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+    const int ib = (int)(t % a.nbra), ik = (int)(t / a.nbra);
+    const PairInfo bra = a.bra_pairs[a.bra_idx[ib]], ket = a.ket_pairs[a.ket_idx[ik]];
+    const double AB[3] = {bra.ABx, bra.ABy, bra.ABz}, CD[3] = {0.0, 0.0, 0.0};
+    const double AC[3] = {bra.Ax - ket.Ax, bra.Ay - ket.Ay, bra.Az - ket.Az};
+    double acc[ACC];
+    md_quartet<ACC>(s, PrimTable{a.bra_prims + bra.pp_off}, bra.npp, PrimTable{a.ket_prims + ket.pp_off}, ket.npp, AB, CD,
+                    AC, 0.0, a.boys, acc);
+    md_store<ACC>(s, acc, 1.0);
+    const long long col0 = a.bra_col[ib];
+    for (int x = threadIdx.x; x < s.nab * s.ncd; x += blockDim.x) {
+      const int k = x / s.nab, ab = x % s.nab, i = ab / c.nb, j = ab % c.nb;
+      if (bra.same && j > i) continue;
+      const long long col = bra.same ? col0 + i * (i + 1) / 2 + j : col0 + ab;
+      a.out[(long long)(ket.ao_a + k) * a.ld + col] = s.out[k * s.os + ab];
+    }
+  }
+}
+
 int md_resident_blocks(const void* kern, int threads, size_t smem) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
@@ -547,6 +575,19 @@ int md_blocks_per_sm(int la, int lb, int lc, int ld) {
 bool md_class_ok(int la, int lb, int lc, int ld) {
   return la >= 0 && lb >= 0 && lc >= 0 && ld >= 0 && la <= kMDLMax && lb <= kMDLMax && lc <= kMDLMax &&
          ld <= kMDLMax;
+}
+
+cudaError_t launch_df3c_md(int la, int lb, int lc, const Df3cArgs& args, cudaStream_t st) {
+  const long long total = (long long)args.nbra * args.nket;
+  if (total <= 0) return cudaSuccess;
+  const MDClass c = md_class(la, lb, lc, 0);
+  const size_t smem = md_smem(c, false);
+  auto kern = HFG_MD_KERNEL(df3c_md_kernel, c);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int nt = md_threads(c);
+  kern<<<(unsigned)std::min<long long>(total, md_resident_blocks((const void*)kern, nt, smem)), nt, smem, st>>>(c, args);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,

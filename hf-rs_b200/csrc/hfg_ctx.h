@@ -190,6 +190,10 @@ struct hfg_ctx {
   PlanMap plans, other_plans[3];
   hfg_jk_stats last{};
 
+  // cuBLAS / cuSOLVER handles (handles.h) and their release
+  void *blas = nullptr, *solver = nullptr;
+  void (*free_handles)(hfg_ctx*) = nullptr;
+
   ~hfg_ctx();
 };
 

@@ -35,6 +35,22 @@ def test_tensor_core_exchange_over_occupied_counts(cluster, nocc, mma, tol):
     assert np.array_equal(K, K.T)
 
 
+def test_three_centre_integrals_agree_between_launch_sizes():
+    # a monomer's launches are small (lanes per combination, a block per
+    # combination in the high classes); inside the cluster the same shells are
+    # part of launches large enough for one lane each
+    atoms = water_cluster(9)
+    big, small = CartesianBasis.build(atoms, "cc-pvdz"), CartesianBasis.build(atoms[:3], "cc-pvdz")
+    auxb, auxs = CartesianBasis.build(atoms, AUX), CartesianBasis.build(atoms[:3], AUX)
+    cb, cs = Context(big), Context(small)
+    want = cs.df_three_center(auxs)
+    got = cb.df_three_center(auxb)[:auxs.n, :want.shape[1]]
+    # 1e-14 relative per integral, cancellation within a contraction up to 1e2
+    assert np.max(np.abs(got - want)) < 1e-12 * np.max(np.abs(want))
+    cb.close()
+    cs.close()
+
+
 @pytest.mark.parametrize("n_occ,frozen", [(1, 0), (10, 0), (10, 3), (33, 1), (49, 0)])
 @pytest.mark.parametrize("storage", [HFG_DF_FP64, HFG_DF_FP32])
 def test_ri_mp2_matches_its_definition_on_the_transformed_factor(n_occ, frozen, storage):
