@@ -94,6 +94,58 @@ __global__ void scale_cols_kernel(double* __restrict__ V, const double* __restri
   V[t] *= rsqrt(w[first + col]);
 }
 
+// The scalars of one SCF iteration, in one launch and one copy to the host
+// (a library dot or amax call each, with its own synchronisation, cost 0.3 ms
+// an iteration at n = 50): per spin (blockIdx.y) and quantity (blockIdx.x),
+//   0: P.H   1: P.F   2: max|E|   3: |P - Pprev|^2   4 + i: E_i.E (history i,
+// or E itself).  blockIdx.z reduces its share of the elements; the host adds
+// the shares in order.  Longer histories take a launch per kScalarHist
+// vectors, of which the first alone has quantities 0 to 3.
+constexpr int kScalarParts = 64, kScalarHist = 32;
+struct ScalarArgs {
+  const double *P, *Pprev, *H, *F, *E, *Eh;
+  int slot[kScalarHist];            // history slots (of Eh), -1: E
+  int lead;                         // 4: with quantities 0 to 3, else 0
+  long long nn, elen, estride;      // E of spin s at E + s elen; slot t, spin s at Eh + (t nspin + s) estride
+  int nspin;
+  double* out;                      // [nspin][quantities][parts]
+};
+__global__ void __launch_bounds__(256) scf_scalars_kernel(const ScalarArgs a) {
+  const int hi = (int)blockIdx.x - a.lead, what = hi < 0 ? (int)blockIdx.x : 4, sp = blockIdx.y;
+  const bool err = what == 2 || what == 4;
+  const long long len = err ? a.elen : a.nn;
+  const long long per = (len + gridDim.z - 1) / gridDim.z, i0 = blockIdx.z * per, i1 = min(len, i0 + per);
+  const double* x = err ? a.E + sp * a.elen : a.P + sp * a.nn;
+  const double* y = x;
+  if (what == 0) y = a.H;
+  if (what == 1) y = a.F + sp * a.nn;
+  if (what == 3) y = a.Pprev + sp * a.nn;
+  if (what == 4 && a.slot[hi] >= 0) y = a.Eh + ((long long)a.slot[hi] * a.nspin + sp) * a.estride;
+  double s = 0.0;
+  for (long long i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    if (what == 2) {
+      s = fmax(s, fabs(x[i]));
+    } else if (what == 3) {
+      const double d = x[i] - y[i];
+      s = fma(d, d, s);
+    } else {
+      s = fma(x[i], y[i], s);
+    }
+  }
+  __shared__ double part[8];
+  for (int off = 16; off > 0; off >>= 1) {
+    const double o = __shfl_xor_sync(0xffffffffu, s, off);
+    s = what == 2 ? fmax(s, o) : s + o;
+  }
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = part[0];
+    for (int k = 1; k < 8; ++k) t = what == 2 ? fmax(t, part[k]) : t + part[k];
+    a.out[((size_t)sp * gridDim.x + blockIdx.x) * gridDim.z + blockIdx.z] = t;
+  }
+}
+
 inline unsigned nblk(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 // Gaussian elimination with partial pivoting (first maximum wins), None
@@ -678,6 +730,8 @@ int hfg_scf(hfg_ctx* ctx, const hfg_scf_opts* o, hfg_scf_result* res, double* P_
   CK(Fh.alloc((long long)hist * nspin * nn));
   CK(Eh.alloc((long long)hist * nspin * elen));
   CK(Fp.alloc(std::max(nn, elen) * 1));
+  DevBuf<double> scal;
+  CK(scal.alloc((size_t)nspin * (5 + hist) * kScalarParts));
   CK(s.evals.alloc(std::max(n, m) * 2));
   const int nocc[2] = {na, nb};
   const double occ_scale = uhf ? 1.0 : 2.0;
@@ -850,23 +904,45 @@ int hfg_scf(hfg_ctx* ctx, const hfg_scf_opts* o, hfg_scf_result* res, double* P_
     else RK(fock(refining ? jo64 : jo));
     phase(0);
     if (refining) ++refine_done;
-    e_tot = energy() + e_nuc;
+    for (int sp = 0; sp < nspin; ++sp) RK(error(sp, E.p + sp * elen_eff));
+    // the history this iteration's error joins (the oldest vector drops out of
+    // a full one), then the error itself
+    std::vector<int> kept(slot.begin() + (count < hist ? 0 : 1), slot.end());
+    kept.push_back(-1);
+    double sc[4] = {0.0, 0.0, 0.0, 0.0};   // P.H and P.F over spins; max|E| and |dP|^2 of the largest spin
+    std::vector<double> edot(kept.size());  // E_i.E over spins
+    {
+      const int parts = (int)std::max<long long>(1, std::min<long long>(kScalarParts, nn / 16384));
+      std::vector<double> h((size_t)nspin * (4 + kept.size()) * parts);
+      size_t off = 0;
+      for (size_t i0 = 0; i0 < kept.size(); i0 += kScalarHist) {
+        const int nh = (int)std::min<size_t>(kScalarHist, kept.size() - i0);
+        ScalarArgs sa{P.p, Pprev.p, s.H.p, F.p, E.p, Eh.p, {}, i0 == 0 ? 4 : 0, nn, elen_eff, elen, nspin, scal.p + off};
+        for (int i = 0; i < nh; ++i) sa.slot[i] = kept[i0 + i];
+        scf_scalars_kernel<<<dim3((unsigned)(sa.lead + nh), (unsigned)nspin, (unsigned)parts), 256, 0, ctx->stream>>>(sa);
+        CK(cudaGetLastError());
+        off += (size_t)nspin * (sa.lead + nh) * parts;
+      }
+      CK(cudaMemcpyAsync(h.data(), scal.p, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+      CK(cudaStreamSynchronize(ctx->stream));
+      const double* v = h.data();
+      for (size_t i0 = 0; i0 < kept.size(); i0 += kScalarHist) {
+        const int lead = i0 == 0 ? 4 : 0, nh = (int)std::min<size_t>(kScalarHist, kept.size() - i0);
+        for (int sp = 0; sp < nspin; ++sp)
+          for (int q = 0; q < lead + nh; ++q) {
+            double t = 0.0;
+            for (int k = 0; k < parts; ++k, ++v) t = q == 2 && lead ? std::max(t, *v) : t + *v;
+            if (q >= lead) edot[i0 + q - lead] += t;
+            else if (q < 2) sc[q] += t;
+            else sc[q] = std::max(sc[q], t);
+          }
+      }
+    }
+    e_tot = 0.5 * (sc[0] + sc[1]) + e_nuc;
     const double de = std::fabs(e_tot - prev_e);
     prev_e = e_tot;
-    double en = 0.0;
-    for (int sp = 0; sp < nspin; ++sp) {
-      RK(error(sp, E.p + sp * elen_eff));
-      en = std::max(en, s.maxabs(E.p + sp * elen_eff, elen_eff));
-    }
     // rmsd of the density change (src/matrix.rs:150-159), max over spins
-    double dr = 0.0;
-    for (int sp = 0; sp < nspin; ++sp) {
-      CK(cudaMemcpyAsync(s.tmp1.p, P.p + sp * nn, nn * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-      axpby_kernel<<<nblk(nn), 256, 0, ctx->stream>>>(s.tmp1.p, Pprev.p + sp * nn, -1.0, 1.0, nn);
-      double nr = 0.0;
-      cublasDnrm2(s.blas, (int)nn, s.tmp1.p, 1, &nr);
-      dr = std::max(dr, nr / std::sqrt((double)nn));
-    }
+    const double en = sc[2], dr = std::sqrt(sc[3]) / std::sqrt((double)nn);
     if (o->verbose) fprintf(stderr, "hfg scf %3d  E = %.12f  dE = %.3e  |e| = %.3e  dP = %.3e  %s\n", it, e_tot, de, en, dr,
                            refining ? "fp64" : "mixed");
     if (it > 1 && de < o->energy_tol && en < o->residual_tol && dr < o->density_tol &&
@@ -907,14 +983,7 @@ int hfg_scf(hfg_ctx* ctx, const hfg_scf_opts* o, hfg_scf_result* res, double* P_
     std::vector<double> Bn((size_t)k * k);
     // rebuild the overlap matrix in slot order (previous entries reused)
     {
-      std::vector<double> newrow(k);
-      for (int i = 0; i < k; ++i) {
-        double d = 0.0;
-        for (int sp = 0; sp < nspin; ++sp)
-          d += s.dot(Eh.p + ((long long)slot[i] * nspin + sp) * elen, Eh.p + ((long long)sl * nspin + sp) * elen,
-                     elen_eff);
-        newrow[i] = d;
-      }
+      const std::vector<double>& newrow = edot;
       // previous matrix in previous order: entries for slots shared with the new order
       const int kprev = (int)std::sqrt((double)Bm.size());
       for (int i = 0; i < k - 1; ++i)
