@@ -385,10 +385,42 @@ static int build_pairs(hfg_ctx* ctx) {
   return HFG_OK;
 }
 
+// A ket of the entry with the most primitive pairs (the first, but for
+// entries merged over pair classes, where the longest lane counts).
+static int longest_ket(const hfg_ctx* ctx, const JKEntry& x) {
+  const int c0 = ctx->h_pairs[x.k_lo].cls, c1 = ctx->h_pairs[x.k_hi - 1].cls;
+  int best = x.k_lo;
+  for (int c = c0 + 1; c <= c1; ++c)
+    if (ctx->h_pairs[ctx->classes[c].first].npp > ctx->h_pairs[best].npp) best = ctx->classes[c].first;
+  return best;
+}
+
 // Nominal primitive quartets per lane of one warp task of an entry.
 static double entry_cost(const hfg_ctx* ctx, const JKEntry& x) {
   return (double)prim_range(0, 1, ctx->h_pairs[x.bra].npp, x.slice, 0).count *
-         prim_range(0, 1, ctx->h_pairs[x.k_lo].npp, x.slice, 16).count;
+         prim_range(0, 1, ctx->h_pairs[longest_ket(ctx, x)].npp, x.slice, 16).count;
+}
+
+// Joins a bra's ket ranges over pair classes that differ in their primitive
+// counts alone (they follow one another in the pair table) where that saves
+// warp tasks.  The classes of a small molecule hold a few pairs each: one
+// water in 6-31G* has 28 (ss) pairs in 6 classes, a task with 1 to 12 of 32
+// lanes at work for each.  The kets between the ranges are below the Schwarz
+// threshold, which the kernels test per lane.
+static void merge_entries(Launch& L) {
+  std::stable_sort(L.entries.begin(), L.entries.end(), [](const JKEntry& x, const JKEntry& y) {
+    return x.bra != y.bra ? x.bra < y.bra : x.k_lo < y.k_lo;
+  });
+  auto tasks = [](int lo, int hi) { return (hi - lo + 31) / 32; };
+  std::vector<JKEntry> out;
+  for (const JKEntry& x : L.entries) {
+    if (!out.empty() && out.back().bra == x.bra &&
+        tasks(out.back().k_lo, x.k_hi) < tasks(out.back().k_lo, out.back().k_hi) + tasks(x.k_lo, x.k_hi))
+      out.back().k_hi = x.k_hi;
+    else
+      out.push_back(x);
+  }
+  L.entries.swap(out);
 }
 
 // Whether a launch runs on the block-per-quartet engine instead of its
@@ -430,7 +462,7 @@ static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sm
   std::vector<JKEntry> out;
   bool any = false;
   for (const JKEntry& x : L.entries) {
-    const PairInfo &b = ctx->h_pairs[x.bra], &k = ctx->h_pairs[x.k_lo];
+    const PairInfo &b = ctx->h_pairs[x.bra], &k = ctx->h_pairs[longest_ket(ctx, x)];
     if ((double)b.npp * k.npp <= target) {
       out.push_back(x);
       continue;
@@ -575,6 +607,15 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   for (auto& L : plan->launches) {
     L.st = ctx->stream;
     L.coop = coop_launch(L, use);
+    // A batch fills the chip, so that idle lanes cost time (48 molecules of one
+    // to four waters in 6-31G*: 4.58 -> 3.75 ms); the tasks of one small molecule have
+    // SMs to themselves, where a merged task waits for its longest lane (one
+    // water in cc-pVDZ 203 -> 307 us, two 453 -> 515 us).
+    if (precision == HFG_FP64 && use == kPlanBatch) {
+      const size_t before = L.entries.size();
+      merge_entries(L);
+      if (L.entries.size() < before) plan->sliced = true;
+    }
     if (slice_entries(ctx, L, prim_eps, sms, use)) plan->sliced = true;
     // Work-queue steps.  Entries are ordered by the nominal cost of one of
     // their warp tasks (bra x ket primitive pairs, before primitive

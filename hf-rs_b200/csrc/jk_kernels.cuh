@@ -310,9 +310,12 @@ __device__ __forceinline__ void jk_step(const JKLaunchArgs& a, long long c, int 
           const PrimRange rb = prim_range(bra.rec_off, bra.rec_stride, bra.npp, slice, 0);
           const PrimRange rk = prim_range(ket.rec_off, ket.rec_stride, ket.npp, slice, 16);
           const Rec* __restrict__ br = RecOf<T>::get(a) + rb.off;
-          const Rec* __restrict__ kr = RecOf<T>::get(a) + rk.off;
+          // (a ket with fewer primitive pairs than its entry has ket slices may
+          // have none in this slice)
+          const int ko = sizeof(T) == 4 || rk.count > 0 ? rk.off : ket.rec_off;
+          const Rec* __restrict__ kr = RecOf<T>::get(a) + ko;
           const float* __restrict__ bb = a.pbound + rb.off;
-          const float* __restrict__ kb = a.pbound + rk.off;
+          const float* __restrict__ kb = a.pbound + ko;
           const int nb = rb.count, nk = rk.count, bs = rb.stride, ks = rk.stride;
           // screening products in FP32 (bounds are stored as floats; count_kernel
           // evaluates the same products)
