@@ -595,13 +595,14 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
     return std::make_tuple(x.la + x.lb + x.lc + x.ld, x.fp32) > std::make_tuple(y.la + y.lb + y.lc + y.ld, y.fp32);
   });
   // The launches of a large plan fill the GPU one by one, and more of them at
-  // once only share its caches (eight streams / four: (H2O)5 in cc-pVDZ 1,925
-  // / 2,051 us, (H2O)12 in 6-31G* 3,109 / 3,178 us; (H2O)12 in cc-pVDZ 21.8 /
-  // 21.4 ms, mixed UHF (H2O)24 73.3 / 70.8 ms): four from 2.5e7
-  // quartets, (H2O)12 in cc-pVDZ.
+  // once only share its caches (eight / four / three streams: (H2O)5 in
+  // cc-pVDZ 1.83 / 2.12 / 2.19 ms and (H2O)12 in 6-31G* 2.96 / 3.23 / 3.17;
+  // (H2O)12 in cc-pVDZ 21.8 / 21.4 / 21.0, mixed (H2O)18 27.2 / 26.5 / 26.3 and
+  // mixed UHF (H2O)24 73.3 / 73.2 / 70.5).  The line lies between the second
+  // and the third, of about 1.4e7 and 3e7 quartets.
   double quartets = 0.0;
   for (const Launch& L : plan->launches) quartets += L.quartets;
-  if (quartets > 2.5e7) plan->streams = 4;
+  if (quartets > 1.8e7) plan->streams = 3;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   for (auto& L : plan->launches) {
