@@ -58,7 +58,8 @@ constexpr unsigned long long kCholWaitNs = 2000000000ull;
 
 struct CholState {
   unsigned arrived;     // blocks that have reached the barrier, over all steps
-  int bad;              // a residual diagonal fell below -1e-10 scale
+  int bad[2];           // a residual diagonal fell below -1e-10 scale (by the step that reads it: a block may
+                        // be one step ahead of another) or no pivot was found
   int status;           // 0 running, 1 done, 2 budget, 3 a bounded wait ran out
   long long rank;
   double residual;
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kCholThreads) chol_kernel(const CholArgs a) {
     if (tid == 0) __stcg(bm + blockIdx.x, m);
     target += G;
     if (!chol_barrier(a.st, target, &ok)) return;
-    if (*(volatile int*)&a.st->bad) {
+    if (*(volatile int*)&a.st->bad[rank & 1]) {
       if (blockIdx.x == 0 && tid == 0) a.st->rank = rank;
       return;
     }
@@ -160,6 +161,10 @@ __global__ void __launch_bounds__(kCholThreads) chol_kernel(const CholArgs a) {
     for (int b = tid; b < G; b += kCholThreads)
       if (__ldcg(bm + b) >= bound && b < first) first = b;
     const long long owner = block_min(first, redl);
+    if (owner == none) {  // an infinite diagonal: nothing compares with its bound
+      if (blockIdx.x == 0 && tid == 0) a.st->bad[0] = 1;
+      return;
+    }
     first = none;
     const long long o1 = min(a.np, (owner + 1) * a.per);
     for (long long k = owner * a.per + tid; k < o1; k += kCholThreads)
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(kCholThreads) chol_kernel(const CholArgs a) {
       }
     const long long pivot = block_min(first, redl);
     if (pivot == none) {  // no finite diagonal is left
-      if (blockIdx.x == 0 && tid == 0) a.st->bad = 1;
+      if (blockIdx.x == 0 && tid == 0) a.st->bad[0] = 1;
       return;
     }
     const double maximum = __ldcg(diag + pivot);
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(kCholThreads) chol_kernel(const CholArgs a) {
         const double r = k == pivot ? root : v / root;
         __stcg(row + k, r);
         const double d = __ldcg(diag + k) - r * r;
-        if (d < -1e-10 * a.scale) a.st->bad = 1;
+        if (d < -1e-10 * a.scale) a.st->bad[(rank + 1) & 1] = 1;
         __stcg(next + k, fmax(d, 0.0));
       }
       __syncthreads();
@@ -291,7 +296,7 @@ extern "C" int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, h
       return set_error(ctx, HFG_ERR_TIMEOUT, "pivoted Cholesky ERI decomposition: a bounded wait ran out");
     if (h.status == 2)
       return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: factor storage exceeds the memory budget");
-    if (h.bad)
+    if (h.bad[0] || h.bad[1])
       return set_error(ctx, HFG_ERR_INTEGRAL, "pivoted Cholesky ERI decomposition: nonpositive residual Coulomb diagonal");
     rank = h.rank;
     maxres = h.residual;
