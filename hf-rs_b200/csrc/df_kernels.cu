@@ -186,7 +186,9 @@ cudaError_t launch_df_map(const int2* colmn, long long ncol, int n, int* map, cu
 // zeros included, in coalesced rows that gather from B_q through the map
 // (a B_q row is re-read from L2); a scatter from the packed columns writes
 // each pair to two far places in pieces of a sector and needs the chunk
-// cleared first.  The block's threads keep their map entries over its Q.
+// cleared first (J/K on the FP64 factor of (H2O)9, with this unpack and
+// without: 0.81 and 1.22 ms).  The block's threads keep their map entries over
+// its Q.
 template <typename TO, typename TI>
 __global__ void __launch_bounds__(256) df_unpack_kernel(const TI* __restrict__ B, long long ldb,
                                                         const int* __restrict__ map, int q0, int qc, int n,

@@ -196,7 +196,8 @@ extern "C" int hfg_df_mp2(hfg_df* df, const double* C, const double* eps, int m,
   const int n = df->n, qc = chunk_size(df, (size_t)n * no), rank = df->rank;
   // occupied orbitals per block: about 768 rows of V, so that a block's GEMM
   // fills the GPU while the block's own upper triangle of pairs (computed
-  // for nothing) stays small
+  // for nothing) stays small ((H2O)6 in cc-pVDZ: 1.5 ms, 3.2 with a GEMM and a
+  // synchronisation per occupied orbital and the whole transform)
   const int ib = std::max(1, std::min(no, 768 / nv));
   const int nblk = (no + ib - 1) / ib;
   constexpr int kParts = 32;  // partial sums per occupied orbital
