@@ -446,10 +446,12 @@ static bool coop_launch(const Launch& L, PlanUse use) {
 // like a quartet, and the digestion bounds the slices from below at 32
 // primitive quartets (8 / 16 / 32 / 64: one water in cc-pVDZ 214 / 219 / 214 /
 // 263 us, (H2O)5 1,943 / 1,867 / 1,826 / 1,786, (H2O)5 in STO-3G, UHF, 216 /
-// 135 / 100 / 124).  Batched builds fill the GPU with whole molecules and
+// 135 / 100 / 124), and at a twentieth of a warp's share of the whole plan's
+// work (without / with: (H2O)5 in cc-pVDZ 1,810 / 1,756 us, mixed (H2O)24 in
+// STO-3G 1,063 / 1,041; at a fifth (H2O)5 takes 1,903).  Batched builds fill the GPU with whole molecules and
 // slice from 128.  FP32 launches hold
 // quartets with few primitive quartets left and are not sliced.
-static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sms, PlanUse use) {
+static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sms, PlanUse use, double work) {
   const bool generic = L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
   if (L.fp32 || use == kPlanWhole || (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld))) return false;
   const bool block = use == kPlanGrad || (use == kPlanJK && (L.coop || generic));  // a block per quartet
@@ -458,7 +460,7 @@ static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sm
   double target;
   if (block) target = std::max(2.0, total / ((double)sms * md_blocks_per_sm(L.la, L.lb, L.lc, L.ld)));
   else if (use == kPlanBatch) target = std::max(128.0, total / ((double)sms * 16));
-  else target = std::max(32.0, total / ((double)sms * 16));
+  else target = std::max({32.0, total / ((double)sms * 16), 0.05 * work / ((double)sms * 16)});
   std::vector<JKEntry> out;
   bool any = false;
   for (const JKEntry& x : L.entries) {
@@ -605,6 +607,11 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   if (quartets > 1.8e7) plan->streams = 3;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  // nominal primitive quartets per lane of all launches that run on lanes
+  double work = 0.0;
+  for (const Launch& L : plan->launches)
+    if (!coop_launch(L, use))
+      for (const JKEntry& x : L.entries) work += entry_cost(ctx, x) * ((x.k_hi - x.k_lo + 31) / 32);
   for (auto& L : plan->launches) {
     L.st = ctx->stream;
     L.coop = coop_launch(L, use);
@@ -617,7 +624,7 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
       merge_entries(L);
       if (L.entries.size() < before) plan->sliced = true;
     }
-    if (slice_entries(ctx, L, prim_eps, sms, use)) plan->sliced = true;
+    if (slice_entries(ctx, L, prim_eps, sms, use, work)) plan->sliced = true;
     // Work-queue steps.  Entries are ordered by the nominal cost of one of
     // their warp tasks (bra x ket primitive pairs, before primitive
     // screening), most expensive first, so that the cheap tasks form the
