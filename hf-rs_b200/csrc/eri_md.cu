@@ -30,6 +30,7 @@
 #include "jk_dispatch.h"
 #include "eri_prim.cuh"
 #include "md_coop.cuh"
+#include "smem_limit.h"
 
 namespace hfg {
 
@@ -547,7 +548,11 @@ int md_resident_blocks(const void* kern, int threads, size_t smem) {
 // the kernel instantiation of a class: two items per thread up to 128 items
 // (md_threads), five beyond
 bool md_small(const MDClass& c) { return md_items(c) <= 128; }
-#define HFG_MD_KERNEL(name, c) (md_small(c) ? name<8> : name<kMDAcc>)
+template <auto Small, auto Large>
+auto md_kernel(const MDClass& c, cudaError_t& e) {
+  e = md_small(c) ? raise_smem_limit<Small>() : raise_smem_limit<Large>();
+  return md_small(c) ? Small : Large;
+}
 
 }  // namespace
 
@@ -582,8 +587,8 @@ cudaError_t launch_df3c_md(int la, int lb, int lc, const Df3cArgs& args, cudaStr
   if (total <= 0) return cudaSuccess;
   const MDClass c = md_class(la, lb, lc, 0);
   const size_t smem = md_smem(c, false);
-  auto kern = HFG_MD_KERNEL(df3c_md_kernel, c);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaSuccess;
+  auto kern = md_kernel<df3c_md_kernel<8>, df3c_md_kernel<kMDAcc>>(c, e);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c);
   kern<<<(unsigned)std::min<long long>(total, md_resident_blocks((const void*)kern, nt, smem)), nt, smem, st>>>(c, args);
@@ -596,8 +601,8 @@ cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimP
   if (count <= 0) return cudaSuccess;
   const MDClass c = md_class(la, lb, la, lb);
   const size_t smem = md_smem(c, false);
-  auto kern = HFG_MD_KERNEL(schwarz_md_kernel, c);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaSuccess;
+  auto kern = md_kernel<schwarz_md_kernel<8>, schwarz_md_kernel<kMDAcc>>(c, e);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c), grid = std::min(count, md_resident_blocks((const void*)kern, nt, smem));
   kern<<<(unsigned)grid, nt, smem, st>>>(c, pairs, prims, first, count, boys, out, prim_mode);
@@ -609,8 +614,8 @@ cudaError_t launch_quartet_md(int la, int lb, int lc, int ld, const PairInfo* pa
   if (!md_class_ok(la, lb, lc, ld)) return cudaErrorInvalidValue;
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = md_smem(c, false);
-  auto kern = HFG_MD_KERNEL(quartet_md_kernel, c);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaSuccess;
+  auto kern = md_kernel<quartet_md_kernel<8>, quartet_md_kernel<kMDAcc>>(c, e);
   if (e != cudaSuccess) return e;
   kern<<<1, md_threads(c), smem, st>>>(c, pairs, prims, boys, out);
   return cudaGetLastError();
@@ -625,8 +630,8 @@ cudaError_t launch_eri_packed_md(int la, int lb, int lc, int ld, const JKEntry* 
   if (nwarps > 0x7fffffffLL) return cudaErrorInvalidValue;
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = md_smem(c, false);
-  auto kern = HFG_MD_KERNEL(eri_packed_md_kernel, c);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaSuccess;
+  auto kern = md_kernel<eri_packed_md_kernel<8>, eri_packed_md_kernel<kMDAcc>>(c, e);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c);
   const long long grid = std::min<long long>(nwarps * 32, md_resident_blocks((const void*)kern, nt, smem));
@@ -639,10 +644,9 @@ cudaError_t launch_jk_md(int la, int lb, int lc, int ld, const JKLaunchArgs& a, 
   if (a.nchunks <= 0) return cudaSuccess;
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = md_smem(c, true);
-  const bool small = md_small(c);
-  auto kern = a.jobs ? (small ? jk_md_kernel<8, true> : jk_md_kernel<kMDAcc, true>)
-                     : (small ? jk_md_kernel<8, false> : jk_md_kernel<kMDAcc, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaSuccess;
+  auto kern = a.jobs ? md_kernel<jk_md_kernel<8, true>, jk_md_kernel<kMDAcc, true>>(c, e)
+                     : md_kernel<jk_md_kernel<8, false>, jk_md_kernel<kMDAcc, false>>(c, e);
   if (e != cudaSuccess) return e;
   const int nt = md_threads(c);
   const long long units = a.nchunks * 32;

@@ -32,6 +32,7 @@
 #include "grad_gen.cuh"
 #include "jk_dispatch.h"
 #include "md_coop.cuh"
+#include "smem_limit.h"
 
 namespace hfg {
 
@@ -464,7 +465,7 @@ cudaError_t launch_lane(const GradArgs& a, long long ntasks, cudaStream_t st) {
   auto kern = grad_lane_kernel<LA, LB, LC, LD>;
   const size_t smem = boys_smem_bytes<double>() + (size_t)(kLaneThreads / 32) * NABCD * lane_slots(NABCD) * 8 +
                       (a.natom <= kLaneGradAtoms ? (size_t)a.natom * 24 : 0);
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t err = raise_smem_limit<grad_lane_kernel<LA, LB, LC, LD>>();
   if (err != cudaSuccess) return err;
   // every task has at most 32 units of one warp each
   const long long want = (ntasks * 32 + kLaneThreads / 32 - 1) / (kLaneThreads / 32);
@@ -521,7 +522,7 @@ cudaError_t launch_eri_gradient(int la, int lb, int lc, int ld, const JKLaunchAr
 #undef HFG_CASE
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = coop_smem(c);
-  cudaError_t err = cudaFuncSetAttribute(grad_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t err = raise_smem_limit<grad_coop_kernel>();
   if (err != cudaSuccess) return err;
   const long long grid =
       std::min<long long>(j.nwarps * 32, resident_blocks((const void*)grad_coop_kernel, kCoopThreads, smem));

@@ -14,6 +14,7 @@
 #include "grad_gen.cuh"
 #include "hfg_ctx.h"
 #include "md_coop.cuh"
+#include "smem_limit.h"
 
 namespace hfg {
 
@@ -539,7 +540,7 @@ static cudaError_t launch_oneint_grad(const OneGradArgs& a, cudaStream_t st) {
   auto kern = oneint_grad_kernel<LA, LB>;
   const size_t smem = boys_smem_bytes<double>() +
                       (3 * (size_t)a.natom + 2 * ncart(LA) * ncart(LB) * (kOneGradThreads / 32)) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = raise_smem_limit<oneint_grad_kernel<LA, LB>>();
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
