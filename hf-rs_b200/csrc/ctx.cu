@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <numeric>
 
 #include "boys.cuh"
@@ -438,29 +439,58 @@ static bool coop_launch(const Launch& L, PlanUse use) {
   return !L.fp32 && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
 }
 
-// Splits the entries whose lanes (or, on the block-per-quartet engine, whose
-// blocks) would walk more primitive quartets than their share of the launch
-// over sms x 16 warps: a (ss|ss) quartet of 8 x 8 primitives each walks 4,096
-// one after another, 1.2 ms, while a molecule of a few atoms fills a fraction
-// of the GPU.  J and K are linear in the integrals, so a slice is digested
-// like a quartet, and the digestion bounds the slices from below at 32
-// primitive quartets (8 / 16 / 32 / 64: one water in cc-pVDZ 214 / 219 / 214 /
-// 263 us, (H2O)5 1,943 / 1,867 / 1,826 / 1,786, (H2O)5 in STO-3G, UHF, 216 /
-// 135 / 100 / 124), and at a twentieth of a warp's share of the whole plan's
-// work (without / with: (H2O)5 in cc-pVDZ 1,810 / 1,756 us, mixed (H2O)24 in
-// STO-3G 1,063 / 1,041; at a fifth (H2O)5 takes 1,903).  Batched builds fill the GPU with whole molecules and
-// slice from 128.  FP32 launches hold
-// quartets with few primitive quartets left and are not sliced.
-static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, int sms, PlanUse use, double work) {
+// Nominal work of a launch's whole entries: primitive quartets a lane walks
+// over its warp tasks, a block over its quartets, and of the longest quartet.
+struct LaunchWork {
+  double lanes = 0.0, blocks = 0.0, most = 0.0;
+};
+static LaunchWork launch_work(const hfg_ctx* ctx, const Launch& L) {
+  LaunchWork w;
+  for (const JKEntry& x : L.entries) {
+    const double c = entry_cost(ctx, x);
+    w.lanes += c * ((x.k_hi - x.k_lo + 31) / 32);
+    w.blocks += c * (x.k_hi - x.k_lo);
+    w.most = std::max(w.most, c);
+  }
+  return w;
+}
+
+// Primitive quartets above which a quartet is sliced, so that its lane (or,
+// on the block-per-quartet engine, its block) does not walk more than its
+// share of the launch over sms x 16 warps: a (ss|ss) quartet of 8 x 8
+// primitives each walks 4,096 one after another, 1.2 ms, while a molecule of
+// a few atoms fills a fraction of the GPU.  J and K are linear in the
+// integrals, so a slice is digested like a quartet, and the digestion bounds
+// the slices from below at 32 primitive quartets (8 / 16 / 32 / 64: one water
+// in cc-pVDZ 214 / 219 / 214 / 263 us, (H2O)5 1,943 / 1,867 / 1,826 / 1,786,
+// (H2O)5 in STO-3G, UHF, 216 / 135 / 100 / 124), and at a twentieth of a
+// warp's share of the whole plan's work (without / with: (H2O)5 in cc-pVDZ
+// 1,810 / 1,756 us, mixed (H2O)24 in STO-3G 1,063 / 1,041; at a fifth (H2O)5
+// takes 1,903).  Batched builds fill the GPU with whole molecules and slice
+// from 128.  FP32 launches hold quartets with few primitive quartets left and
+// are not sliced.  `work` is the lanes' work of the whole plan.
+static double slice_target(const Launch& L, const LaunchWork& w, int sms, PlanUse use, double work) {
   const bool generic = L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
-  if (L.fp32 || use == kPlanWhole || (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld))) return false;
-  const bool block = use == kPlanGrad || (use == kPlanJK && (L.coop || generic));  // a block per quartet
-  double total = 0.0;
-  for (const JKEntry& x : L.entries) total += entry_cost(ctx, x) * (block ? x.k_hi - x.k_lo : (x.k_hi - x.k_lo + 31) / 32);
-  double target;
-  if (block) target = std::max(2.0, total / ((double)sms * md_blocks_per_sm(L.la, L.lb, L.lc, L.ld)));
-  else if (use == kPlanBatch) target = std::max(128.0, total / ((double)sms * 16));
-  else target = std::max({32.0, total / ((double)sms * 16), 0.05 * work / ((double)sms * 16)});
+  if (L.fp32 || use == kPlanWhole || (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld)))
+    return std::numeric_limits<double>::infinity();
+  const double share = (double)sms * 16;
+  if (use == kPlanGrad || (use == kPlanJK && (coop_launch(L, use) || generic)))  // a block per quartet
+    return std::max(2.0, w.blocks / ((double)sms * md_blocks_per_sm(L.la, L.lb, L.lc, L.ld)));
+  if (use == kPlanBatch) return std::max(128.0, w.lanes / share);
+  return std::max({32.0, w.lanes / share, 0.05 * work / share});
+}
+
+// Whether a J/K plan's launch, whole quartets and all, is what `use` would
+// make of it.  FP64 batches join ket ranges (merge_entries), which is looked
+// for in their own plans only.
+static bool launch_serves(const Launch& L, const LaunchWork& w, int sms, int precision, PlanUse use) {
+  if (use == kPlanBatch && precision == HFG_FP64) return false;
+  if (use == kPlanWhole && coop_launch(L, kPlanWhole) != coop_launch(L, kPlanJK)) return false;
+  return w.most <= slice_target(L, w, sms, use, 0.0);
+}
+
+// Splits the entries above `target` primitive quartets.
+static bool slice_entries(const hfg_ctx* ctx, Launch& L, double prim_eps, double target) {
   std::vector<JKEntry> out;
   bool any = false;
   for (const JKEntry& x : L.entries) {
@@ -509,7 +539,7 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   if (tile <= 0) tile = 64;
   auto key = std::make_tuple(thr, precision == HFG_MIXED ? mixed : 0.0, prim_eps, precision, tile);
   auto it = ctx->plans.find(key);
-  if (it != ctx->plans.end() && (use == kPlanJK || !it->second->sliced)) {
+  if (it != ctx->plans.end() && (use == kPlanJK || it->second->serves[use - 1])) {
     out = it->second.get();
     return HFG_OK;
   }
@@ -607,12 +637,15 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
   if (quartets > 1.8e7) plan->streams = 3;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  // nominal primitive quartets per lane of all launches that run on lanes
+  // nominal work of each launch, and of all launches that run on lanes
+  std::vector<LaunchWork> lwork;
   double work = 0.0;
-  for (const Launch& L : plan->launches)
-    if (!coop_launch(L, use))
-      for (const JKEntry& x : L.entries) work += entry_cost(ctx, x) * ((x.k_hi - x.k_lo + 31) / 32);
+  for (const Launch& L : plan->launches) {
+    lwork.push_back(launch_work(ctx, L));
+    if (!coop_launch(L, use)) work += lwork.back().lanes;
+  }
   for (auto& L : plan->launches) {
+    LaunchWork& lw = lwork[&L - plan->launches.data()];
     L.st = ctx->stream;
     L.coop = coop_launch(L, use);
     // A batch fills the chip, so that idle lanes cost time (48 molecules of one
@@ -620,11 +653,13 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
     // SMs to themselves, where a merged task waits for its longest lane (one
     // water in cc-pVDZ 203 -> 307 us, two 453 -> 515 us).
     if (precision == HFG_FP64 && use == kPlanBatch) {
-      const size_t before = L.entries.size();
       merge_entries(L);
-      if (L.entries.size() < before) plan->sliced = true;
+      lw = launch_work(ctx, L);
     }
-    if (slice_entries(ctx, L, prim_eps, sms, use, work)) plan->sliced = true;
+    const double target = slice_target(L, lw, sms, use, work);
+    const bool sliced = lw.most > target && slice_entries(ctx, L, prim_eps, target);
+    for (int u = kPlanWhole; u < kPlanUses; ++u)
+      plan->serves[u - 1] = plan->serves[u - 1] && !sliced && launch_serves(L, lw, sms, precision, (PlanUse)u);
     // Work-queue steps.  Entries are ordered by the nominal cost of one of
     // their warp tasks (bra x ket primitive pairs, before primitive
     // screening), most expensive first, so that the cheap tasks form the
@@ -1021,14 +1056,17 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
 
 hfg_ctx::~hfg_ctx() {
   if (free_handles) free_handles(this);
-  for (auto* map : {&plans, &other_plans[0], &other_plans[1], &other_plans[2]})
-    for (auto& kv : *map)
+  auto free_plans = [](PlanMap& map) {
+    for (auto& kv : map)
       for (auto& L : kv.second->launches) {
         if (L.d_entries) cudaFreeAsync(L.d_entries, L.st);
         if (L.d_prefix) cudaFreeAsync(L.d_prefix, L.st);
         if (L.d_chunk) cudaFreeAsync(L.d_chunk, L.st);
         if (L.d_cstart) cudaFreeAsync(L.d_cstart, L.st);
       }
+  };
+  free_plans(plans);
+  for (auto& map : other_plans) free_plans(map);
   for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
   // every device buffer is released here, before the context's stream is
   // destroyed (their frees are ordered on it)

@@ -54,6 +54,7 @@ struct Launch {
 // fill the GPU: coarser slices), the gradient (whose lane kernel splits the
 // primitive quartets by itself: slices for the other classes only).
 enum PlanUse { kPlanJK = 0, kPlanWhole = 1, kPlanBatch = 2, kPlanGrad = 3 };
+constexpr int kPlanUses = 4;
 
 // side streams on which a J/K build's class launches (and the other sets of
 // independent launches) run next to the context stream: a small molecule's
@@ -64,7 +65,8 @@ struct Plan {
   std::vector<Launch> launches;
   hfg_jk_stats stats{};  // nominal counts until `counted`
   double thr = 0.0, prim_eps = 0.0;
-  bool sliced = false;   // some entries are slices of quartets
+  // whether a J/K plan is also what each other use (PlanUse - 1) would make
+  bool serves[kPlanUses - 1] = {true, true, true};
   int streams = 1 + kJKSideStreams;  // concurrent launches of a build
   bool counted = false;  // exact shell/primitive-quartet counts made (on the first stats request)
 };
@@ -184,10 +186,10 @@ struct hfg_ctx {
   hfg::DevBuf<float> d_D32;  // FP32 copies of a build's densities (3 n^2)
 
   // launch plans by (Schwarz, FP32 and primitive thresholds, precision, tile)
-  // and, where the J/K plan slices quartets, those sliced otherwise for the
-  // other uses (PlanUse - 1)
+  // and, where the J/K plan does not serve them, those of the other uses
+  // (PlanUse - 1)
   using PlanMap = std::map<std::tuple<double, double, double, int, int>, std::unique_ptr<hfg::Plan>>;
-  PlanMap plans, other_plans[3];
+  PlanMap plans, other_plans[hfg::kPlanUses - 1];
   hfg_jk_stats last{};
 
   // cuBLAS / cuSOLVER handles (handles.h) and their release

@@ -96,3 +96,16 @@ def test_packed_tensor_and_gradient_after_a_sliced_build():
     assert np.max(np.abs(ctx.eri_packed(1e-12) - ref)) < 1e-12
     assert np.max(np.abs(ctx.eri_gradient(P) - g0)) < 1e-12 * np.max(np.abs(g0))
     ctx.close()
+
+
+def test_packed_tensor_does_not_depend_on_an_earlier_build():
+    # 666 (dd|dd) quartets of one primitive each: the J/K plan slices nothing
+    # and takes its generated kernel there, the packed tensor's the block engine
+    atoms = [("He", (1.6 * (i % 2), 1.7 * (i // 2 % 2), 1.5 * (i // 4) + 0.1 * i)) for i in range(8)]
+    basis = CartesianBasis(atoms, {"HE": [(2, np.array([0.8]), np.array([1.0]), None),
+                                          (0, np.array([1.1]), np.array([1.0]), None)]})
+    fresh, used = Context(basis), Context(basis)
+    used.jk(rand_sym(basis.n, 6))
+    assert np.array_equal(fresh.eri_packed(1e-12), used.eri_packed(1e-12))
+    fresh.close()
+    used.close()
