@@ -433,10 +433,12 @@ static void merge_entries(Launch& L) {
 // 108.9 / 109.4 / 113.2 / 113.1 ms.  A batched launch has its quartets spread
 // over many short queues and gains up to 2,000 (4.78 ms at 500, 4.57 at 2,000,
 // 4.96 at 8,000 for 48 molecules of 1 to 4 waters), and so does the packed
-// tensor, whose kernels do not split the heavy classes' quartets.
+// tensor, whose kernels do not split the heavy classes' quartets.  In a
+// deterministic build one thread of the engine digests every quartet (one
+// water in cc-pVDZ 283 ms with it and with slices, 129 with neither).
 static bool coop_launch(const Launch& L, PlanUse use) {
   const double limit = use == kPlanBatch || use == kPlanWhole ? 2000.0 : 500.0;
-  return !L.fp32 && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
+  return !L.fp32 && use != kPlanSerial && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
 }
 
 // Nominal work of a launch's whole entries: primitive quartets a lane walks
@@ -471,7 +473,8 @@ static LaunchWork launch_work(const hfg_ctx* ctx, const Launch& L) {
 // are not sliced.  `work` is the lanes' work of the whole plan.
 static double slice_target(const Launch& L, const LaunchWork& w, int sms, PlanUse use, double work) {
   const bool generic = L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
-  if (L.fp32 || use == kPlanWhole || (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld)))
+  if (L.fp32 || use == kPlanWhole || use == kPlanSerial ||
+      (use == kPlanGrad && eri_gradient_splits(L.la, L.lb, L.lc, L.ld)))
     return std::numeric_limits<double>::infinity();
   const double share = (double)sms * 16;
   if (use == kPlanGrad || (use == kPlanJK && (coop_launch(L, use) || generic)))  // a block per quartet
@@ -485,7 +488,7 @@ static double slice_target(const Launch& L, const LaunchWork& w, int sms, PlanUs
 // for in their own plans only.
 static bool launch_serves(const Launch& L, const LaunchWork& w, int sms, int precision, PlanUse use) {
   if (use == kPlanBatch && precision == HFG_FP64) return false;
-  if (use == kPlanWhole && coop_launch(L, kPlanWhole) != coop_launch(L, kPlanJK)) return false;
+  if ((use == kPlanWhole || use == kPlanSerial) && coop_launch(L, use) != coop_launch(L, kPlanJK)) return false;
   return w.most <= slice_target(L, w, sms, use, 0.0);
 }
 
@@ -877,7 +880,8 @@ int jk_device_locked(hfg_ctx* ctx, const hfg_jk_opts* opts, int nspin, const dou
   if (ctx->batcher && nspin == 1 && nshards == 1 && dPs == dPt && !o.deterministic)
     return batcher_submit(ctx->batcher, ctx, o, dPt, dJ, dK);
   Plan* plan = nullptr;
-  int rc = build_plan(ctx, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile, kPlanJK, plan);
+  int rc = build_plan(ctx, o.schwarz_threshold, o.mixed_threshold, o.prim_threshold, o.precision, o.tile,
+                      o.deterministic ? kPlanSerial : kPlanJK, plan);
   if (rc != HFG_OK) return rc;
   const size_t nn = (size_t)ctx->n * ctx->n;
   HFG_CUDA(ctx, ctx->d_Jacc.alloc(nn));

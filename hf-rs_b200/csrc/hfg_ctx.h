@@ -52,9 +52,10 @@ struct Launch {
 // What a plan's entries are sliced for: one J/K build, consumers that need
 // every quartet whole (the packed tensor), a batched build (many molecules
 // fill the GPU: coarser slices), the gradient (whose lane kernel splits the
-// primitive quartets by itself: slices for the other classes only).
-enum PlanUse { kPlanJK = 0, kPlanWhole = 1, kPlanBatch = 2, kPlanGrad = 3 };
-constexpr int kPlanUses = 4;
+// primitive quartets by itself: slices for the other classes only), and a
+// deterministic build (one warp, or one block, runs the queue: no slices).
+enum PlanUse { kPlanJK = 0, kPlanWhole = 1, kPlanBatch = 2, kPlanGrad = 3, kPlanSerial = 4 };
+constexpr int kPlanUses = 5;
 
 // side streams on which a J/K build's class launches (and the other sets of
 // independent launches) run next to the context stream: a small molecule's
@@ -66,7 +67,7 @@ struct Plan {
   hfg_jk_stats stats{};  // nominal counts until `counted`
   double thr = 0.0, prim_eps = 0.0;
   // whether a J/K plan is also what each other use (PlanUse - 1) would make
-  bool serves[kPlanUses - 1] = {true, true, true};
+  bool serves[kPlanUses - 1] = {true, true, true, true};
   int streams = 1 + kJKSideStreams;  // concurrent launches of a build
   bool counted = false;  // exact shell/primitive-quartet counts made (on the first stats request)
 };

@@ -100,13 +100,19 @@ extern "C" int hfg_jk_device_noalloc(hfg_ctx* ctx, const hfg_jk_opts* opts, int 
   std::lock_guard<std::mutex> lk(ctx->mu);
   const auto key = std::make_tuple(o.schwarz_threshold, o.precision == HFG_MIXED ? o.mixed_threshold : 0.0,
                                    o.prim_threshold, o.precision, o.tile > 0 ? o.tile : 64);
+  // the plan that hfg_jk_device would take, else any with this key
   auto it = ctx->plans.find(key);
   bool found = it != ctx->plans.end();
-  for (auto& m : ctx->other_plans) {
-    if (found) break;
-    it = m.find(key);
-    found = it != m.end();
-  }
+  auto look = [&](hfg_ctx::PlanMap& m) {
+    const auto f = m.find(key);
+    if (f == m.end()) return;
+    it = f;
+    found = true;
+  };
+  if (o.deterministic && !(found && it->second->serves[hfg::kPlanSerial - 1]))
+    look(ctx->other_plans[hfg::kPlanSerial - 1]);
+  for (auto& m : ctx->other_plans)
+    if (!found) look(m);
   if (!found)
     return hfg::set_error(ctx, HFG_ERR_INVALID_INPUT,
                           "hfg_jk_device_noalloc: no launch plan for these options on this context; call hfg_jk or "

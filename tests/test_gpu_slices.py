@@ -109,3 +109,28 @@ def test_packed_tensor_does_not_depend_on_an_earlier_build():
     assert np.array_equal(fresh.eri_packed(1e-12), used.eri_packed(1e-12))
     fresh.close()
     used.close()
+
+
+def test_deterministic_builds_take_whole_quartets():
+    # one warp (or block) runs a deterministic build's queue: its plan has no
+    # slices, so it agrees to the bit with a build on the packed tensor's plan
+    # (s, p and f shells: no class that only one of the two gives the block engine)
+    import ctypes
+
+    import torch
+    sh = [(l, np.array([2.4, 1.1, 0.5]), np.array([0.4, 0.5, 0.3]), None) for l in (0, 1, 3)]
+    basis = CartesianBasis(ATOMS[:2], {"HE": sh})
+    n, det = basis.n, JKOptions.make(deterministic=True)
+    ctx, other = Context(basis), Context(basis)
+    P = rand_sym(n, 7)
+    J, K = ctx.jk(P, opts=det)
+    other.eri_packed(1e-12)
+    dP = torch.from_numpy(P).cuda()
+    dJ, dK = torch.empty_like(dP), torch.empty_like(dP)
+    torch.cuda.synchronize()
+    assert other.lib.hfg_jk_device_noalloc(other.h, ctypes.byref(det), 1, dP.data_ptr(), dP.data_ptr(), dJ.data_ptr(),
+                                           dK.data_ptr()) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(dJ.cpu().numpy(), J) and np.array_equal(dK.cpu().numpy(), K[0])
+    ctx.close()
+    other.close()
