@@ -550,33 +550,16 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
     } else {
       CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, st));
     }
-  }
-  // The stored FP32 / BF16 factor with FP64 accumulation (J reads it twice and
-  // is bound by HBM; the density is not rounded) runs on a side stream beside
-  // the exchange, whose kernels leave half the bandwidth unused; the context
-  // stream waits for it on every path out of here.
-  struct Join {
-    hfg_ctx* c = nullptr;
-    ~Join() {
-      if (!c) return;
-      cudaEventRecord(c->ev_join[0], c->side[0]);
-      cudaStreamWaitEvent(c->stream, c->ev_join[0], 0);
-    }
-  } join;
-  cudaStream_t js = st;
-  if (df->storage != HFG_DF_FP64) {
-    CK(ctx->ensure_side_streams());
-    CK(cudaEventRecord(ctx->ev_fork, st));
-    CK(cudaStreamWaitEvent(ctx->side[0], ctx->ev_fork, 0));
-    js = ctx->side[0];
-    join.c = ctx;
+  } else {
+    // the stored FP32 / BF16 factor with FP64 accumulation (J is
+    // memory-bound; the density is not rounded)
     const bool bf = df->storage == HFG_DF_BF16;
-    if (rank == 0) CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, js));
+    if (rank == 0) CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, st));
     CK(launch_df_j(bf ? 2 : 1, bf ? (const void*)(df->B16.p + (size_t)q_lo * ncol) : (const void*)(df->B32.p + (size_t)q_lo * ncol), ncol, rank, df->pvec.p,
-                   df->gam.p, df->jcol.p, js));
+                   df->gam.p, df->jcol.p, st));
   }
-  CK(cudaMemsetAsync(dJ, 0, nn * 8, js));
-  CK(launch_unpack_j(df->jcol.p, df->colmn.p, ncol, n, dJ, js));
+  CK(cudaMemsetAsync(dJ, 0, nn * 8, st));
+  CK(launch_unpack_j(df->jcol.p, df->colmn.p, ncol, n, dJ, st));
 
   // K on the tensor cores: this library's tcgen05 kernels (df_umma.cu).
   // HFG_DF_K_CUBLAS=1 selects the cuBLAS GEMMs below instead, kept only to
