@@ -630,14 +630,22 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
     return std::make_tuple(x.la + x.lb + x.lc + x.ld, x.fp32) > std::make_tuple(y.la + y.lb + y.lc + y.ld, y.fp32);
   });
   // The launches of a large plan fill the GPU one by one, and more of them at
-  // once only share its caches (eight / four / three streams: (H2O)5 in
-  // cc-pVDZ 1.83 / 2.12 / 2.19 ms and (H2O)12 in 6-31G* 2.96 / 3.23 / 3.17;
-  // (H2O)12 in cc-pVDZ 21.8 / 21.4 / 21.0, mixed (H2O)18 27.2 / 26.5 / 26.3 and
-  // mixed UHF (H2O)24 73.3 / 73.2 / 70.5).  The line lies between the second
-  // and the third, of about 1.4e7 and 3e7 quartets.
-  double quartets = 0.0;
-  for (const Launch& L : plan->launches) quartets += L.quartets;
-  if (quartets > 1.8e7) plan->streams = 3;
+  // once only share its caches.  The line is in nominal McMurchie-Davidson
+  // flops (before primitive screening), FP32 ones for a quarter, which puts
+  // FP64 and mixed plans of any basis on one scale.  Eight / three streams, ms:
+  //   0.3e11  FP64 (H2O)12 in 6-31G*        2.39 / 2.57
+  //   1.0e11  mixed (H2O)24 in 6-31G*       9.76 / 9.97
+  //   1.8e11  mixed (H2O)31 in 6-31G*      17.79 / 17.86
+  //   2.0e11  mixed (H2O)12 in cc-pVDZ      7.50 / 8.20   FP64 (H2O)9   8.81 / 8.90
+  //   2.6e11  FP64 (H2O)10                 11.6  / 11.5
+  //   3.7e11  mixed (H2O)14                12.72 / 12.80
+  //   3.8e11  FP64 (H2O)11                 16.5  / 16.1
+  //   5.0e11  FP64 (H2O)12                 21.5  / 21.0
+  //   5.7e11  mixed (H2O)16                18.6  / 18.4
+  //   8.5e11  mixed (H2O)18                27.1  / 26.2
+  // (a line by the number of quartets, at 1.8e7, took mixed plans to three
+  // streams far too early: mixed UHF (H2O)16 in 6-31G* 6.05 ms, 5.5 on eight)
+  if (st.wmd_flops_fp64 + 0.25 * st.wmd_flops_fp32 > 3.5e11) plan->streams = 3;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   // nominal work of each launch, and of all launches that run on lanes
