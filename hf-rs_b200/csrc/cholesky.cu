@@ -279,14 +279,17 @@ extern "C" int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, h
     int sms = 148, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chol_kernel, kCholThreads, 0));
-    // one block per SM, at least one tile of columns each
-    const int blocks = (int)std::max<long long>(1, std::min<long long>(per_sm > 0 ? sms : 1, (np + kCholCols - 1) / kCholCols));
+    // whole tiles of columns per block, as few as blocks on every SM can
+    // share, and no block without columns (n_p = 5,050: 79 blocks of two
+    // tiles; every block joins the barrier of each step)
+    const long long most = per_sm > 0 ? sms : 1;
+    long long per = (np + most - 1) / most;
+    per = (per + kCholCols - 1) / kCholCols * kCholCols;
+    const int blocks = (int)((np + per - 1) / per);
     CK(bmax.alloc(2 * (size_t)blocks));
     CK(state.alloc(1));
     CK(dpiv.alloc((size_t)cap));
     CK(cudaMemsetAsync(state.p, 0, sizeof(CholState), st));
-    long long per = (np + blocks - 1) / blocks;
-    per = (per + kCholCols - 1) / kCholCols * kCholCols;
     CholArgs a{V.p, df->B64.p, diag.p, bmax.p, state.p, dpiv.p, np, cap, per, threshold, scale, (double)budget};
     void* args[] = {&a};
     CK(cudaLaunchCooperativeKernel((const void*)chol_kernel, dim3((unsigned)blocks), dim3(kCholThreads), args, 0, st));

@@ -9,8 +9,8 @@ from hfgpu.lib import DFTensor
 pytestmark = pytest.mark.gpu
 
 
-# 28 pairs (less than one tile of 32 columns), 325, and 5,050 (several tiles
-# in some of 148 blocks, none in others)
+# 28 pairs (less than one tile of 32 columns), 325 (a tile per block, the last
+# short), and 5,050 (two tiles per block, more than one on each of 148 SMs)
 @pytest.mark.parametrize("nw,basis,threshold", [(1, "sto-3g", 1e-8), (1, "cc-pvdz", 1e-7), (4, "cc-pvdz", 1e-4)])
 def test_factor_reproduces_the_supermatrix_within_its_residual(nw, basis, threshold):
     ctx = Context(CartesianBasis.build(water_cluster(nw), basis))
