@@ -550,16 +550,43 @@ int df_jk_device(hfg_df* df, const double* dC, int nocc, double* dJ, double* dK,
     } else {
       CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, st));
     }
-  } else {
-    // the stored FP32 / BF16 factor with FP64 accumulation (J is
-    // memory-bound; the density is not rounded)
-    const bool bf = df->storage == HFG_DF_BF16;
-    if (rank == 0) CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, st));
-    CK(launch_df_j(bf ? 2 : 1, bf ? (const void*)(df->B16.p + (size_t)q_lo * ncol) : (const void*)(df->B32.p + (size_t)q_lo * ncol), ncol, rank, df->pvec.p,
-                   df->gam.p, df->jcol.p, st));
   }
-  CK(cudaMemsetAsync(dJ, 0, nn * 8, st));
-  CK(launch_unpack_j(df->jcol.p, df->colmn.p, ncol, n, dJ, st));
+  // The stored FP32 / BF16 factor with FP64 accumulation (J reads it twice and
+  // is bound by HBM; the density is not rounded).  Up to kJBeside AOs it runs
+  // on a side stream beside the exchange, which leaves bandwidth unused, and
+  // the context stream waits for it on every path out of here.  Beside / before
+  // a BF16 exchange of the FP32 factor, ms: (H2O)20 in STO-3G (n = 140) 0.59 /
+  // 0.70, (H2O)14 in 6-31G* (266) 0.79 / 0.90, in cc-pVDZ (H2O)12 (300) 0.75 /
+  // 0.81, (H2O)24 (600) 2.86 / 3.05, (H2O)32 (800) 6.21 / 6.32, (H2O)40 (1,000)
+  // 12.2 / 12.8, (H2O)48 (1,200) 21.4 / 21.5, (H2O)64 (1,600) 51.1 / 51.4 and
+  // (H2O)80 106.1 / 106.1; FP64 arithmetic, (H2O)10: 1.00 / 1.15.  Above the
+  // line it would gain nothing and stretch the exchange's reported time
+  // (hfg_df_last_stats; (H2O)64: 51 instead of 45).
+  constexpr int kJBeside = 1100;
+  struct Join {
+    hfg_ctx* c = nullptr;
+    ~Join() {
+      if (!c) return;
+      cudaEventRecord(c->ev_join[0], c->side[0]);
+      cudaStreamWaitEvent(c->stream, c->ev_join[0], 0);
+    }
+  } join;
+  cudaStream_t js = st;
+  if (df->storage != HFG_DF_FP64) {
+    if (n <= kJBeside) {
+      CK(ctx->ensure_side_streams());
+      CK(cudaEventRecord(ctx->ev_fork, st));
+      CK(cudaStreamWaitEvent(ctx->side[0], ctx->ev_fork, 0));
+      js = ctx->side[0];
+      join.c = ctx;
+    }
+    const bool bf = df->storage == HFG_DF_BF16;
+    if (rank == 0) CK(cudaMemsetAsync(df->jcol.p, 0, ncol * 8, js));
+    CK(launch_df_j(bf ? 2 : 1, bf ? (const void*)(df->B16.p + (size_t)q_lo * ncol) : (const void*)(df->B32.p + (size_t)q_lo * ncol), ncol, rank, df->pvec.p,
+                   df->gam.p, df->jcol.p, js));
+  }
+  CK(cudaMemsetAsync(dJ, 0, nn * 8, js));
+  CK(launch_unpack_j(df->jcol.p, df->colmn.p, ncol, n, dJ, js));
 
   // K on the tensor cores: this library's tcgen05 kernels (df_umma.cu).
   // HFG_DF_K_CUBLAS=1 selects the cuBLAS GEMMs below instead, kept only to

@@ -362,7 +362,9 @@ int hfg_cholesky_eri(hfg_ctx* ctx, double threshold, size_t budget, hfg_df** out
  * No counterpart in hf-rs.  Device time (ms) of the exchange (K) of the last
  * tensor-core hfg_df_jk on this factor, the tensor-core flops it executed
  * (both GEMMs, zero tiles skipped, lower triangle of K only), and the share
- * of the 128-row tiles of the unpacked B_Q that hold any stored AO pair.
+ * of the 128-row tiles of the unpacked B_Q that hold any stored AO pair.  Up to
+ * 1,100 AOs J is built beside the exchange, whose time then includes what J
+ * takes of the memory bandwidth; above, the exchange runs alone.
  */
 int hfg_df_last_stats(hfg_df* df, double* k_ms, double* k_flops, double* tiles_fraction);
 
