@@ -1690,7 +1690,7 @@ int eri_packed_locked(hfg_ctx* ctx, double thr, double* d_out, size_t len) {
     const bool md = L.coop || L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
     le = md ? launch_eri_packed_md(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0], L.prefix[1],
                                    ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p, ctx->d_pbound.p,
-                                   ctx->d_boys64.p, ctx->d_expt64.p, d_out, ls)
+                                   ctx->d_boys64.p, d_out, ls)
             : launch_eri_packed(L.la, L.lb, L.lc, L.ld, L.d_entries, L.d_prefix, (int)L.prefix[0], L.prefix[1],
                                 ctx->d_pairs.p, ctx->d_pairQ.p, thr, ctx->d_rec64.p, ctx->d_boys64.p,
                                 ctx->d_expt64.p, d_out, ls);

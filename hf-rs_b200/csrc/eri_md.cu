@@ -596,7 +596,7 @@ cudaError_t launch_df3c_md(int la, int lb, int lc, const Df3cArgs& args, cudaStr
 }
 
 cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,
-                              const double* boys, const double* expt, double* out, int prim_mode, cudaStream_t st) {
+                              const double* boys, double* out, int prim_mode, cudaStream_t st) {
   if (!md_class_ok(la, lb, la, lb)) return cudaErrorInvalidValue;
   if (count <= 0) return cudaSuccess;
   const MDClass c = md_class(la, lb, la, lb);
@@ -610,7 +610,7 @@ cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimP
 }
 
 cudaError_t launch_quartet_md(int la, int lb, int lc, int ld, const PairInfo* pairs, const PrimPair* prims,
-                              const double* boys, const double* expt, double* out, cudaStream_t st) {
+                              const double* boys, double* out, cudaStream_t st) {
   if (!md_class_ok(la, lb, lc, ld)) return cudaErrorInvalidValue;
   const MDClass c = md_class(la, lb, lc, ld);
   const size_t smem = md_smem(c, false);
@@ -624,7 +624,7 @@ cudaError_t launch_quartet_md(int la, int lb, int lc, int ld, const PairInfo* pa
 cudaError_t launch_eri_packed_md(int la, int lb, int lc, int ld, const JKEntry* entries, const long long* prefix,
                                  int nentries, long long nwarps, const PairInfo* pairs, const double* pairQ,
                                  double thr, const PrimRec64* rec, const float* pbound, const double* boys,
-                                 const double* expt, double* out, cudaStream_t st) {
+                                 double* out, cudaStream_t st) {
   if (!md_class_ok(la, lb, lc, ld)) return cudaErrorInvalidValue;
   if (nwarps <= 0) return cudaSuccess;
   if (nwarps > 0x7fffffffLL) return cudaErrorInvalidValue;

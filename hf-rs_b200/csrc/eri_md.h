@@ -20,13 +20,13 @@ MDClass md_class(int la, int lb, int lc, int ld);
 bool md_class_ok(int la, int lb, int lc, int ld);
 
 cudaError_t launch_schwarz_md(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,
-                              const double* boys, const double* expt, double* out, int prim_mode, cudaStream_t st);
+                              const double* boys, double* out, int prim_mode, cudaStream_t st);
 cudaError_t launch_quartet_md(int la, int lb, int lc, int ld, const PairInfo* pairs, const PrimPair* prims,
-                              const double* boys, const double* expt, double* out, cudaStream_t st);
+                              const double* boys, double* out, cudaStream_t st);
 cudaError_t launch_eri_packed_md(int la, int lb, int lc, int ld, const JKEntry* entries, const long long* prefix,
                                  int nentries, long long nwarps, const PairInfo* pairs, const double* pairQ,
                                  double thr, const PrimRec64* rec, const float* pbound, const double* boys,
-                                 const double* expt, double* out, cudaStream_t st);
+                                 double* out, cudaStream_t st);
 // FP64 J/K over the launch's work queue (a.serial: one block, deterministic)
 cudaError_t launch_jk_md(int la, int lb, int lc, int ld, const JKLaunchArgs& a, cudaStream_t st);
 // Blocks of the J/K engine that an SM holds, about (by the class's block size)

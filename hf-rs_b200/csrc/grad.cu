@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kCoopThreads) grad_coop_kernel(MDClass c, cons
   const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
   const float inv_ncd = 1.0f / L.ncd, inv_hcd = 1.0f / L.hcd, inv_hab = 1.0f / L.hab;
   const int SS = R.S * R.S, S1 = R.S;
-  const coop::UnitQueue uq = coop::unit_queue(a.chunk_start, a.nchunks, 0);
+  const coop::UnitQueue uq = coop::unit_queue(a.chunk_start, a.nchunks);
   int e = 0;
   for (;;) {
     __syncthreads();

@@ -72,7 +72,7 @@ cudaError_t launch_jk_batch(int la, int lb, int lc, int ld, bool fp32, bool coop
 cudaError_t launch_schwarz(int la, int lb, const PairInfo* pairs, const PrimPair* prims, int first, int count,
                            const double* boys, const double* expt, double* out, int prim_mode, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
-  if (la > kLMax || lb > kLMax) return launch_schwarz_md(la, lb, pairs, prims, first, count, boys, expt, out, prim_mode, st);
+  if (la > kLMax || lb > kLMax) return launch_schwarz_md(la, lb, pairs, prims, first, count, boys, out, prim_mode, st);
   const int smem = (int)boys_smem_bytes<double>();
   const int block = 64, grid = (count + block - 1) / block;
 #define HFG_CASE(A, B)                                                                             \
@@ -94,7 +94,7 @@ cudaError_t launch_schwarz(int la, int lb, const PairInfo* pairs, const PrimPair
 cudaError_t launch_quartet(int la, int lb, int lc, int ld, const PairInfo* pairs, const PrimPair* prims,
                            const double* boys, const double* expt, double* out, cudaStream_t st) {
   if (la > kLMax || lb > kLMax || lc > kLMax || ld > kLMax)
-    return launch_quartet_md(la, lb, lc, ld, pairs, prims, boys, expt, out, st);
+    return launch_quartet_md(la, lb, lc, ld, pairs, prims, boys, out, st);
   const int smem = (int)boys_smem_bytes<double>();
 #define HFG_CASE(A, B, C, D)                                                    \
   if (la == A && lb == B && lc == C && ld == D) {                               \

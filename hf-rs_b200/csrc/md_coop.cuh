@@ -98,7 +98,7 @@ __host__ __device__ inline int side_nnz(int l1, int l2) {
 
 // One side's run-time dimensions and shared-memory tables.
 struct Side {
-  int l1, l2, n1, n2, nab, nh, nnz, sj, st;  // sj, st: strides of the axis table E[ax][i][j][t]
+  int l1, l2, n1, n2, nab, nh, nnz, st;  // st: stride of j in the axis table E[ax][i][j][t]
   double *E, *D;      // axis tables (D: derivatives with respect to A - B, or null)
   double* prod;       // [nnz] E^{ab}_h
   double* dprod;      // [3][nnz] its derivatives (or null)
@@ -130,7 +130,6 @@ __device__ inline unsigned char* side_carve(Side& s, int l1, int l2, bool deriv,
   s.nh = nherm(l1 + l2);
   s.nnz = side_nnz(l1, l2);
   s.st = l1 + l2 + 1;
-  s.sj = s.st;
   unsigned char* const p0 = p;
   const int na = axis_size(l1, l2);
   s.E = (double*)p;
@@ -395,12 +394,12 @@ struct UnitQueue {
   long long t0, units;
   int per;
 };
-__device__ __forceinline__ UnitQueue unit_queue(const long long* chunk_start, long long nchunks, int serial) {
+__device__ __forceinline__ UnitQueue unit_queue(const long long* chunk_start, long long nchunks) {
   UnitQueue q;
   q.t0 = chunk_start[0];
   q.units = (chunk_start[nchunks] - q.t0) * 32;
   const long long per = q.units / ((long long)gridDim.x * 16);
-  q.per = serial ? 32 : (int)(per < 1 ? 1 : (per > 32 ? 32 : per));
+  q.per = (int)(per < 1 ? 1 : (per > 32 ? 32 : per));
   return q;
 }
 
