@@ -430,12 +430,16 @@ static void merge_entries(Launch& L) {
 // once, however few quartets there are.  Measured on water clusters of 1 to
 // 32 molecules, limits of 0 / 500 / 2,000 / 8,000 quartets: one water 842 /
 // 255 / 257 / 259 us, (H2O)4 1,808 / 1,162 / 1,224 / 1,906 us, mixed (H2O)32
-// 108.9 / 109.4 / 113.2 / 113.1 ms.  A batched launch has its quartets spread
-// over many short queues and gains up to 2,000 (4.78 ms at 500, 4.57 at 2,000,
-// 4.96 at 8,000 for 48 molecules of 1 to 4 waters), and so does the packed
-// tensor, whose kernels do not split the heavy classes' quartets.  In a
-// deterministic build one thread of the engine digests every quartet (one
-// water in cc-pVDZ 283 ms with it and with slices, 129 with neither).
+// 108.9 / 109.4 / 113.2 / 113.1 ms.  The packed tensor, whose kernels do not
+// split the heavy classes' quartets, gains up to 2,000 (Cholesky factors of 1, 2
+// and 3 waters in cc-pVDZ 2.9 / 1.7 / 1.7 / 1.7, 4.8 / 3.2 / 3.1 / 3.1 and 6.6 /
+// 5.8 / 5.0 / 5.3 ms).  A batched launch, its quartets spread over many short
+// queues, does so only where they have few primitives (48 molecules of 1 to 4
+// waters in 6-31G* 3.93 / 3.93 / 3.75 / 4.28 ms; 24 of 1 to 3 in cc-pVDZ 4.31 /
+// 4.45 / 4.47 / 4.85, 64 single ones 1.82 / 1.86 / 2.20 / 2.35): a line by
+// primitive quartets would fit better.  In a deterministic build one thread
+// of the engine digests every quartet (one water in cc-pVDZ 283 ms with it
+// and with slices, 130 with neither).
 static bool coop_launch(const Launch& L, PlanUse use) {
   const double limit = use == kPlanBatch || use == kPlanWhole ? 2000.0 : 500.0;
   return !L.fp32 && use != kPlanSerial && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
@@ -469,8 +473,11 @@ static LaunchWork launch_work(const hfg_ctx* ctx, const Launch& L) {
 // warp's share of the whole plan's work (without / with: (H2O)5 in cc-pVDZ
 // 1,810 / 1,756 us, mixed (H2O)24 in STO-3G 1,063 / 1,041; at a fifth (H2O)5
 // takes 1,903).  Batched builds fill the GPU with whole molecules and slice
-// from 128.  FP32 launches hold quartets with few primitive quartets left and
-// are not sliced.  `work` is the lanes' work of the whole plan.
+// from 128 (32 / 128 / 512: 48 molecules of 1 to 4 waters in 6-31G* 4.12 / 3.75
+// / 3.80 ms, 24 of 1 to 3 in cc-pVDZ 5.46 / 4.47 / 4.57, 64 single ones 3.37 /
+// 2.20 / 2.28, 64 of 1 to 4 in STO-3G 0.75 / 0.63 / 0.54).  FP32 launches hold
+// quartets with few primitive quartets left and are not sliced.  `work` is the
+// lanes' work of the whole plan.
 static double slice_target(const Launch& L, const LaunchWork& w, int sms, PlanUse use, double work) {
   const bool generic = L.la > kLMax || L.lb > kLMax || L.lc > kLMax || L.ld > kLMax;
   if (L.fp32 || use == kPlanWhole || use == kPlanSerial ||
@@ -660,7 +667,8 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
     L.st = ctx->stream;
     L.coop = coop_launch(L, use);
     // A batch fills the chip, so that idle lanes cost time (48 molecules of one
-    // to four waters in 6-31G*: 4.58 -> 3.75 ms); the tasks of one small molecule have
+    // to four waters in 6-31G* 4.58 -> 3.75 ms, 24 of one to three in cc-pVDZ 5.05
+    // -> 4.47, 64 single ones 3.20 -> 2.20); the tasks of one small molecule have
     // SMs to themselves, where a merged task waits for its longest lane (one
     // water in cc-pVDZ 203 -> 307 us, two 453 -> 515 us).
     if (precision == HFG_FP64 && use == kPlanBatch) {

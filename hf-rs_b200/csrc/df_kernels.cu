@@ -146,8 +146,10 @@ cudaError_t launch_df3c(int la, int lb, int lc, Df3cArgs args, cudaStream_t st) 
   const long long total = (long long)args.nbra * args.nket;
   if (total <= 0) return cudaSuccess;
   // the high classes' straight-line code is too long to pass through for few
-  // combinations (factor build and J/K of (H2O)5, 665 auxiliary functions: 15.4
-  // ms with this rule, 17.2 without; 15.3 / 16.6 ms from L = 6 / 4)
+  // combinations (factor build and J/K in cc-pVDZ, limits of 0 / 5,000 /
+  // 20,000 / 80,000 / no limit: one water 3.2 / 2.2 / 2.1 / 2.1 / 2.1 ms, (H2O)4 8.9 /
+  // 8.2 / 8.2 / 8.2 / 8.2, (H2O)6 13.9 / 13.1 / 13.1 / 13.1 / 13.1; from L = 6
+  // as fast as from 5, from L = 4 8% slower)
   if (la + lb + lc >= 5 && total <= 20000) return launch_df3c_md(la, lb, lc, args, st);
   // split the bra's primitive pairs over lanes while there are few
   // combinations, at least 4 per lane

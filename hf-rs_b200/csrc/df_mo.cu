@@ -196,8 +196,10 @@ extern "C" int hfg_df_mp2(hfg_df* df, const double* C, const double* eps, int m,
   const int n = df->n, qc = chunk_size(df, (size_t)n * no), rank = df->rank;
   // occupied orbitals per block: about 768 rows of V, so that a block's GEMM
   // fills the GPU while the block's own upper triangle of pairs (computed
-  // for nothing) stays small ((H2O)6 in cc-pVDZ: 1.5 ms, 3.2 with a GEMM and a
-  // synchronisation per occupied orbital and the whole transform)
+  // for nothing) stays small (one orbital / 256 / 768 / 1,536 rows / all at
+  // once: (H2O)2 in cc-pVDZ 0.33 / 0.25 / 0.22 / 0.23 / 0.23 ms, (H2O)4 in
+  // 6-31G* 0.66 / 0.50 / 0.46 / 0.47 / 0.47, (H2O)6 2.4 / 2.0 / 1.7 / 1.7 /
+  // 1.8, (H2O)9 8.4 / 8.4 / 6.1 / 5.8 / 7.2)
   const int ib = std::max(1, std::min(no, 768 / nv));
   const int nblk = (no + ib - 1) / ib;
   constexpr int kParts = 32;  // partial sums per occupied orbital

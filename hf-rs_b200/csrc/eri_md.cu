@@ -19,7 +19,7 @@
 // so the second, larger contraction runs once per ket primitive pair.  The
 // block is 32 to 512 threads by the size of (ab|cd), and the quartets of a
 // launch are handed out one by one.  What bounds it: shared-memory loads in
-// the two contractions (three per multiply-add) for the large classes, the
+// the two contractions (six for four multiply-adds) for the large classes, the
 // chain of short steps with a barrier each for the small ones.
 #include <cuda_runtime.h>
 

@@ -21,8 +21,9 @@
 // * grad_coop_kernel (the d-rich classes, 4 <= L <= 8): one quartet per
 //   block on the tables of md_coop.cuh.  G is contracted with one side's
 //   coefficients (W, X), those with R (V, U, over the nonzero Hermite
-//   products only), and those with the derivative coefficients: about 46,000
-//   multiply-adds per (dd|dd) primitive quartet and 6 block barriers.
+//   products only), and those with the derivative coefficients: about 53,000
+//   multiply-adds per (dd|dd) primitive quartet (12,000 more for a bra
+//   primitive's first) and 6 block barriers.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -57,7 +57,8 @@ struct KetSoA {
 };
 
 // Work entry of one launch: bra pair and the range of ket pairs [k_lo, k_hi)
-// (global pair indices, kets of one pair class).  `slice` is 0 for whole
+// (global pair indices; kets of one pair class or, in a batch's plans, of
+// neighbouring ones that differ in primitive counts).  `slice` is 0 for whole
 // quartets; else the entry covers one slice of the primitive quartets, bra
 // primitive pairs sb, sb + nb, ... and ket ones sk, sk + nk, ..., with sb,
 // nb, sk, nk in its bytes from the lowest (J and K are linear in the

@@ -242,7 +242,7 @@ __device__ __forceinline__ T run_sum(T v, int lane, int end) {
 }
 
 // One work-queue step of a launch: a warp takes one bra shell pair and up
-// to 32 ket pairs of one pair class per task, one shell quartet per lane.
+// to 32 ket pairs of one entry per task, one shell quartet per lane.
 // Step c holds tasks [chunk_start[c], chunk_start[c + 1]) and chunk_entry[c]
 // is the entry of its first task; later tasks of the step walk the prefix
 // forward.
@@ -290,7 +290,8 @@ __device__ __forceinline__ void jk_step(const JKLaunchArgs& a, long long c, int 
         }
         // the next task usually continues this entry: start fetching its
         // first primitive records (kets of one class have equal primitive
-        // counts and consecutive records, so they start 32 on)
+        // counts and consecutive records, so they start 32 on; in an entry
+        // over several classes the record 32 on may be another ket's)
         constexpr bool kPrefetch = sizeof(T) == 4 ? HFG_JK_PREFETCH_F32 != 0 : HFG_JK_PREFETCH_F64 != 0;
         if (kPrefetch && warp + 1 < t1 && kidx + 32 < ent.k_hi) {
           prefetch_l1(RecOf<T>::get(a) + ket.rec_off + 32);

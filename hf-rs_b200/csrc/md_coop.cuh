@@ -6,8 +6,8 @@
 //             E^{cd}_k R_{h+k}(alpha, P - Q),   h = (t,u,v), alpha = pq/(p+q)
 //
 // * A side (ab) holds the products E^{ab}_h = E_t E_u E_v of its nonzero
-//   Hermite indices only (t <= a_x + b_x and so on: 250 of the 36 x 35
-//   products of (dd), 1,540 of 100 x 84 of (ff)), listed by component pair,
+//   Hermite indices only (t <= a_x + b_x and so on: 336 of the 36 x 35
+//   products of (dd), 1,920 of 100 x 84 of (ff)), listed by component pair,
 //   so every contraction is a sparse sum without index arithmetic.
 // * R is stored in a cube of edge S, so the index of h + k is the sum of two
 //   linear offsets.

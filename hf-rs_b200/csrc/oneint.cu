@@ -1,12 +1,12 @@
 // One-electron integrals S, T, V on the device (needed by the SCF driver).
 //
 // McMurchie-Davidson form, as hf-rs computes them (src/integrals.rs:408-535,
-// :747-793; src/scf.rs:247-271): one thread per Cartesian function pair
-// mu >= nu, looping over primitive pairs; Hermite expansion coefficients
+// :747-793; src/scf.rs:247-271).  S and T: one thread per Cartesian function
+// pair mu >= nu, looping over primitive pairs; Hermite expansion coefficients
 // E_t^{ij} per axis, S = E_0^x E_0^y E_0^z (pi/p)^{3/2}, T from the overlap
-// recursion with lb +- 2, V = -Z 2pi/p sum E_t E_u E_v R_tuv(p, P - C) over
-// nuclei.  Instantiated for shells up to d (LM = 2) and up to f (LM = 3);
-// the kinetic term needs E up to lb + 2.
+// recursion with lb +- 2 (instantiated for shells up to d, LM = 2, and up to
+// f, LM = 3; the kinetic term needs E up to lb + 2).  V = -Z 2pi/p sum E_t E_u
+// E_v R_tuv(p, P - C) over nuclei: one warp per shell pair (nuc_kernel).
 #include <cuda_runtime.h>
 
 #include "boys.cuh"

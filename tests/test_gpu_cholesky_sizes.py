@@ -33,3 +33,16 @@ def test_factor_reproduces_the_supermatrix_within_its_residual(nw, basis, thresh
     with pytest.raises(HfgError, match="budget"):
         DFTensor.cholesky(ctx, threshold, budget=8 * npair * (len(piv) - 1))
     ctx.close()
+
+
+def test_an_infinite_diagonal_is_refused():
+    # a contraction coefficient so large that (ss|ss) overflows: no bound holds
+    # for an infinite residual, so no block owns the pivot
+    basis = CartesianBasis([("He", (0.0, 0.0, 0.0)), ("He", (0.0, 0.0, 1.2))], {"HE": [(0, np.array([0.9]), np.array([1.0]),
+                                                                                      None)]})
+    basis.coefs[0] = 1e80
+    ctx = Context(basis)
+    assert np.isinf(ctx.eri_packed(1e-15)[0])
+    with pytest.raises(HfgError, match="residual Coulomb diagonal"):
+        DFTensor.cholesky(ctx, 1e-6)
+    ctx.close()
