@@ -569,7 +569,8 @@ def measure_df(args, torch):
     The FP64-stored factor with FP64 arithmetic is the reference; the
     FP32-stored factor runs the exchange on the tensor cores (this library's
     tcgen05 kernels) with TF32 and with BF16 operands.  Per form: factor
-    build time, J/K wall time, the exchange's device time and executed
+    build time, J/K wall time, the exchange's device time (alone on the GPU
+    above 1,100 AOs, beside J's kernels below: hfg_df_last_stats) and executed
     tensor-core TFLOP/s (both GEMMs, zero tiles skipped, lower triangle of K),
     the reference's algorithmic rate (4 n^2 nocc naux flops), the fraction
     of the measured BF16 tensor peak (TF32 runs at half of it), the error of

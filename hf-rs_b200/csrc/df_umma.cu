@@ -478,9 +478,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // The next Q's values are in flight meanwhile.  The image's 16-byte units are
 // swizzled by row (unit ^ row % 8, as the list's positions are), or the rows
 // of a block, 128 bytes apart, would share their banks.  Elements outside the
-// list stay zero from the start.  Bound by the gathers' sectors through L2:
-// (H2O)24, FP32 factor to BF16 tiles, 1.07 ms, 1.28 in element order, 2.11 with
-// whole tiles and no values in flight.
+// list stay zero from the start.  Bound by the gathers in L1 (its pipe 81%
+// busy, L2 51%, DRAM 46%): (H2O)24, FP32 factor to BF16 tiles, 1.07 ms, 1.28 in
+// element order, 2.11 with whole tiles and no values in flight.
 template <typename TS, typename TD>
 __global__ void __launch_bounds__(256) unpack_tiles_kernel(const TS* __restrict__ B, long long ncol,
                                                            const int* __restrict__ list_off,

@@ -17,7 +17,9 @@
 //   the largest power-of-two group of lanes that its primitive quartets fill,
 //   so a contracted (ss|ss) quartet of 64 x 64 primitive pairs keeps a warp
 //   busy, and quartets of uncontracted shells share one.  These classes hold
-//   nearly all primitive quartets: bound by FP64 latency at 8 warps per SM.
+//   nearly all primitive quartets.  8 warps per SM, which wait on global and
+//   local loads (the generated code's stack) before FP64 results: the FP64
+//   pipe is 10% busy.
 // * grad_coop_kernel (the d-rich classes, 4 <= L <= 8): one quartet per
 //   block on the tables of md_coop.cuh.  G is contracted with one side's
 //   coefficients (W, X), those with R (V, U, over the nonzero Hermite

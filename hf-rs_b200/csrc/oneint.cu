@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(128) oneint_kernel(const OneIntArgs a) {
 // group's sums meet by a butterfly and go to shared memory, and its lanes
 // share the components.  (A thread per function pair, with a four-index R
 // table in local memory per nucleus, took 1.5 ms for two waters in cc-pVDZ.)
+// A small molecule's launches, 46 us each beside one another, wait for their
+// blocks' Boys tables.
 struct NucArgs {
   const PairInfo* pairs;  // of one (la, lb)
   int count;
