@@ -445,15 +445,19 @@ static bool coop_launch(const Launch& L, PlanUse use) {
   return !L.fp32 && use != kPlanSerial && L.la + L.lb + L.lc + L.ld >= 5 && L.quartets <= limit;
 }
 
-// Nominal work of a launch's whole entries: primitive quartets a lane walks
-// over its warp tasks, a block over its quartets, and of the longest quartet.
+// Nominal work of a launch's entries: entry_cost of each, and of all the
+// primitive quartets that a lane walks over its warp tasks, a block over its
+// quartets, and those of the longest quartet.
 struct LaunchWork {
+  std::vector<double> cost;
   double lanes = 0.0, blocks = 0.0, most = 0.0;
 };
 static LaunchWork launch_work(const hfg_ctx* ctx, const Launch& L) {
   LaunchWork w;
+  w.cost.reserve(L.entries.size());
   for (const JKEntry& x : L.entries) {
     const double c = entry_cost(ctx, x);
+    w.cost.push_back(c);
     w.lanes += c * ((x.k_hi - x.k_lo + 31) / 32);
     w.blocks += c * (x.k_hi - x.k_lo);
     w.most = std::max(w.most, c);
@@ -687,12 +691,9 @@ static int build_plan(hfg_ctx* ctx, double thr, double mixed, double prim_eps, i
     // default 64, about eight steps per resident warp, up to 32 warps per
     // SM; the step cost scales with the tile).  Each step's first task and
     // its entry are tabulated, so no warp searches the prefix.
-    std::vector<double> cost;
+    std::vector<double> cost = sliced ? launch_work(ctx, L).cost : std::move(lw.cost);
     {
       const size_t ne = L.entries.size();
-      cost.resize(ne);
-      for (size_t e = 0; e < ne; ++e)
-        cost[e] = entry_cost(ctx, L.entries[e]);
       std::vector<size_t> ord(ne);
       std::iota(ord.begin(), ord.end(), 0);
       std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) { return cost[x] > cost[y]; });
